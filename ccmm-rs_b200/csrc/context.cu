@@ -329,7 +329,7 @@ int32_t ckks_ctx_create(uint32_t log_n, const uint64_t* q, uint32_t L, const uin
     // FP64 networks: primes below 2^50 when both transform halves have at most
     // 2^8 points (four register stages on each side of the exchange)
     const bool f64_shape = ctx->log_n1 <= 8 && ctx->log_n2 <= 8;
-    const size_t fper = 2 * ((size_t)(1u << ctx->log_n1) + (1u << ctx->log_n2) + n);
+    const size_t fper = 2 * ((size_t)(1u << ctx->log_n1) + (1u << ctx->log_n2)) + n;
     size_t n_f64 = 0;
     for (size_t i = 0; i < M; ++i) n_f64 += f64_shape && mod[i] < (1ull << 50);
     std::vector<double2> fhost(fper * n_f64);
@@ -357,8 +357,14 @@ int32_t ckks_ctx_create(uint32_t log_n, const uint64_t* q, uint32_t L, const uin
             fput(ht[i].psiA_inv, &T.fA_inv);
             fput(ht[i].psiB, &T.fB);
             fput(ht[i].psiB_inv, &T.fB_inv);
-            fput(ht[i].mid, &T.fmid);
-            fput(ht[i].midi, &T.fmidi);
+            auto wput = [&](const std::vector<u64>& v, const double** dst) {  // values only, two to an entry
+                double* h = reinterpret_cast<double*>(fhost.data() + foff);
+                for (size_t k = 0; k < v.size(); ++k) h[k] = (double)v[k];
+                *dst = reinterpret_cast<const double*>(ctx->d_ftable_mem + foff);
+                foff += v.size() / 2;
+            };
+            wput(ht[i].mid, &T.fmid);
+            wput(ht[i].midi, &T.fmidi);
         }
         T.q = m;
         barrett_host(m, &T.mu_hi, &T.mu_lo);

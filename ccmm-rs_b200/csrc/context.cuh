@@ -27,7 +27,8 @@ struct NttTab {
     // points): the same tables as (W, fl(W / q)) pairs, q and fl(1 / q)
     int f64;
     double qd, qinv;
-    const double2 *fA, *fA_inv, *fB, *fB_inv, *fmid, *fmidi;
+    const double2 *fA, *fA_inv, *fB, *fB_inv;
+    const double *fmid, *fmidi;  // the twists: W only
 };
 
 constexpr int kMaxAux = 8;  // auxiliary (P) limbs

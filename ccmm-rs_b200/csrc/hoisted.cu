@@ -1288,7 +1288,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
             if ((rc = bounded_decompose_launch(ctx, in0 + (size_t)Lq * n, gn, Lq, k0->base_log, dig.p, flags.p, st,
                                                ct_words)))
                 return rc;
-            if ((rc = ntt_forward_digits_launch(ctx, dig.p, Y.p, D * gn, lqp, LK, st))) return rc;
+            if ((rc = ntt_forward_digits_launch(ctx, dig.p, Y.p, D * gn, lqp, LK, st, k0->base_log))) return rc;
             if (use_tc) {  // the tensor-core MAC takes P b as one more digit: NTT(b) on the Q limbs
                 CKKS_CUDA_TRY(cudaMemcpy2DAsync(Bh.p, b_stride * sizeof(u64), in0, ct_words * sizeof(u64),
                                                 b_stride * sizeof(u64), gn, cudaMemcpyDeviceToDevice, st));

@@ -391,7 +391,7 @@ int32_t rotate_hybrid(ckks_ctx* ctx, const ckks_ksk* key, const u64* ct_in, u64*
         if ((rc = bounded_decompose_launch(ctx, sct + (size_t)Lq * n, m, Lq, key->base_log, dg.p, nullptr, st,
                                            ct_words)))
             return rc;
-        if ((rc = ntt_forward_digits_launch(ctx, dg.p, Y, D * m, lqp, LK, st))) return rc;
+        if ((rc = ntt_forward_digits_launch(ctx, dg.p, Y, D * m, lqp, LK, st, key->base_log))) return rc;
         if ((rc = ntt_forward_launch_map(ctx, sct, s_hat, 2 * m, lq, Lq, st))) return rc;
         if ((rc = ks_mac_launch(ctx, Y, key->d_entries, s_hat, acc, Lq, D, true, 0, 0, st, key->exponent, m,
                                 ct_words)))

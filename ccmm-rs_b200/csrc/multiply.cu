@@ -158,8 +158,8 @@ int32_t relin_core_launch(ckks_ctx* ctx, const ckks_ksk* key, const u64* c2, u64
         if ((rc = dg.alloc((size_t)n * D * N, st))) return rc;
         if ((rc = bounded_decompose_launch(ctx, c2, n, L, key->base_log, dg.p, nullptr, st))) return rc;
         if (relin_fused && ntt_relin_fused_supported(ctx, L))  // digit transforms stay on chip
-            return ntt_relin_fused_launch(ctx, dg.p, Y.p, key->d_entries, acc01, acc01, n, L, D, st);
-        if ((rc = ntt_forward_digits_launch(ctx, dg.p, Y.p, n * D, LimbMap::range(0, L), L, st))) return rc;
+            return ntt_relin_fused_launch(ctx, dg.p, Y.p, key->d_entries, acc01, acc01, n, L, D, st, key->base_log);
+        if ((rc = ntt_forward_digits_launch(ctx, dg.p, Y.p, n * D, LimbMap::range(0, L), L, st, key->base_log))) return rc;
     }
     dim3 g((N + kT - 1) / kT, L, (n + kRelinGroup - 1) / kRelinGroup);
     k_relin_mac<kRelinGroup><<<g, kT, 0, st>>>(Y.p, key->d_entries, acc01, acc01, ctx->d_tabs, (int)n, (int)L, (int)D,

@@ -21,6 +21,7 @@
 // 2^54 skip the conditional subtractions and estimate the Shoup quotient from
 // three 32-bit partial products); outputs are canonical.
 #include <cstdio>
+#include <type_traits>
 
 #include "ntt_core.cuh"
 #include "moddown_f64.cuh"
@@ -34,10 +35,17 @@ constexpr int kMaxThreads = 256;
 // Resident CTAs of kMaxThreads per SM asked of the register allocator: 3 caps a
 // thread at 80 registers, 4 at 64. Tiles of up to 2^8 points fit those caps with
 // at most a few words of spill, and the extra resident warps hide the global
-// loads (forward pass 1 over digits: 1157 -> 953 us for 27 limbs x 64 polys of
-// N = 2^16 at 64 registers; the inverse passes gain about 3 % at 80). 2^9-point
-// tiles spill hundreds of bytes at either cap and keep the compiler's own
-// allocation (a minimum of 0 leaves the count unspecified).
+// loads. 2^9-point tiles spill hundreds of bytes at either cap and keep the
+// compiler's own allocation (a minimum of 0 leaves the count unspecified).
+//
+// What bounds the passes: at N = 2^16 each moves its data once (2.1 GB for 2048
+// limb-polynomials, 323 us at the copy rate) and needs about 80 instructions a point
+// in two dependent halves, so neither DRAM nor the FP64 pipe is full. Issuing a
+// tile's global loads before its twiddle table is staged, column counts as
+// constants, bit reversals split into a constant and a thread's part, 8-byte twist
+// entries and digits taken signed gave, for 2048 limb-polynomials (616 x 27 for the
+// digits): forward pass 1 590 -> 454 us, pass 2 463 -> 395, inverse pass 1 572 ->
+// 476, pass 2 527 -> 476, forward pass 1 of 32-bit digits 5.62 -> 3.98 ms.
 template <int LOG_M>
 constexpr int min_ctas(int want) {
     return LOG_M <= 8 ? want : 0;
@@ -62,6 +70,21 @@ __device__ __forceinline__ u64 lift_digit(i64 d, u64 q, u64 m) {
     return (d < 0 && r) ? q - r : r;
 }
 
+// Bit reversal of R2 g + e (e below R2 = 2^LR2, g below R1 = 2^LR1): brev(e) is a constant
+// of the unrolled loops, so only brev(g) is computed.
+template <int LOG_M>
+__device__ __forceinline__ u32 brev_hi(int e) {
+    using S = Split<LOG_M>;
+    return brev((u32)e, S::LR2) << S::LR1;
+}
+
+// A digit known to lie in [-2^(b-1), 2^(b-1)) with 2^(b-1) <= q: no reduction.
+__device__ __forceinline__ u64 lift_small(i64 d, u64 q) { return d < 0 ? (u64)d + q : (u64)d; }
+// |d| < 2^51 -> double (exact): 2^52 + 2^51 + d has the bits 0x4338.. + d.
+__device__ __forceinline__ double digit_double(i64 d) {
+    return __dsub_rn(__longlong_as_double(d + 0x4338000000000000ll), 6755399441055744.0);
+}
+
 // Stage a small (W, W/q) table of the FP64 networks in shared memory (16-byte
 // entries: one 128-bit shared load per twiddle).
 __device__ __forceinline__ const double2* stage_table_f64(u64* at, const double2* __restrict__ v, int M) {
@@ -83,20 +106,36 @@ __device__ __forceinline__ void stage_table(u64* st, const u64* __restrict__ v, 
 // psi^((2k_a+1-A) j_lo), stored as row j_lo in natural k_a order.
 // kDigits: the input is a signed digit polynomial [D][N] shared by every limb
 // (blockIdx.z = digit), lifted on load (signed_mod, hybrid_rns_galois_key.rs:55-57).
-template <int LOG_M, bool kDigits>
+// Digits below 2^(digit_log - 1) in magnitude, at most q, need no reduction (digit_log 0:
+// unknown): the FP64 network takes them signed.
+// The global loads are issued before the table is staged, so the two latencies overlap;
+// the twist is one 8-byte table entry (its quotient factor is one multiplication).
+template <int LOG_M, bool kDigits, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(4))
 k_fwd1(const void* __restrict__ in_, u64* __restrict__ out,
        const NttTab* __restrict__ tabs, LimbMap lm, int limb_count,
-       int log_b, int log_c) {
+       int log_b, int log_c_, int digit_log) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int limb = blockIdx.y;
     const NttTab& T = tabs[lm(limb)];
     const u64 q = T.q;
     const size_t base = ((size_t)blockIdx.z * limb_count + limb) << (LOG_M + log_b);
     const int c0 = blockIdx.x << log_c;
-    if (LOG_M <= 8 && T.f64) {  // FP64 network: inputs in [0, q), twist output below q in magnitude
+    const bool small = kDigits && digit_log > 0 && digit_log <= 52 && (1ull << (digit_log - 1)) <= q;
+    if (LOG_M <= 8 && T.f64) {  // FP64 network: inputs at most q in magnitude, twist output below 2 q
+        u64 raw[S::R1];
+        const bool act1 = tid < (C << S::LR2);
+        const int c1 = tid & (C - 1), i0 = tid >> log_c;
+        if (act1) {
+            const u64* src = (const u64*)in_ + (kDigits ? (size_t)blockIdx.z << (LOG_M + log_b) : base) + c0 + c1 +
+                             ((size_t)i0 << log_b);
+            const size_t step = (size_t)S::R2 << log_b;
+#pragma unroll
+            for (int e = 0; e < S::R1; ++e) raw[e] = src[e * step];
+        }
         // Phase 2 runs the row group g = tid % R1 in the low lanes, so a warp reads 16
         // different blocks (g << ls) + b of a stage s = LR1 + ls: they are staged at
         // (1 << s) + (b << LR1) + g (consecutive in g) instead of 2^ls entries apart,
@@ -118,37 +157,38 @@ k_fwd1(const void* __restrict__ in_, u64* __restrict__ out,
             return tab[(1u << s) + ((blk & ((1u << ls) - 1)) << S::LR1) + (blk >> ls)];
         };
         __syncthreads();
-        if (tid < (C << S::LR2)) {
-            const int c = tid & (C - 1), i0 = tid >> log_c;
+        if (act1) {
             double x[S::R1];
-            if (kDigits) {
-                const i64* in = (const i64*)in_ + ((size_t)blockIdx.z << (LOG_M + log_b));
+            if (kDigits && small) {
+#pragma unroll
+                for (int e = 0; e < S::R1; ++e) x[e] = digit_double((i64)raw[e]);
+            } else {
 #pragma unroll
                 for (int e = 0; e < S::R1; ++e)
-                    x[e] = nttf::from_u52(lift_digit(in[c0 + c + ((size_t)(i0 + S::R2 * e) << log_b)], q, T.mu_hi));
-            } else {
-                const u64* in = (const u64*)in_ + base;
-#pragma unroll
-                for (int e = 0; e < S::R1; ++e) x[e] = nttf::from_u52(in[c0 + c + ((size_t)(i0 + S::R2 * e) << log_b)]);
+                    x[e] = nttf::from_u52(kDigits ? lift_digit((i64)raw[e], q, T.mu_hi) : raw[e]);
             }
             nttf::ct_stages<S::LR1>(x, 0, 0, twf, qd);
+            double* o = smd + (i0 << log_c);
 #pragma unroll
             for (int e = 0; e < S::R1; ++e)
-                smd[((i0 + S::R2 * e) << log_c) + (c ^ (e & (C - 1)))] = nttf::center(x[e], qd, qinv);
+                o[((S::R2 * e) << log_c) + (c1 ^ (e & (C - 1)))] = nttf::center(x[e], qd, qinv);
         }
         __syncthreads();
         if (tid < (C << S::LR1)) {
             const int g = tid & (S::R1 - 1), c = tid >> S::LR1;
             double y[S::R2];
+            const double* o = smd + ((S::R2 * g) << log_c) + (c ^ (g & (C - 1)));
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) y[e] = smd[((S::R2 * g + e) << log_c) + (c ^ (g & (C - 1)))];
+            for (int e = 0; e < S::R2; ++e) y[e] = o[e << log_c];
             nttf::ct_stages<S::LR2>(y, S::LR1, g, twf2, qd);
-            const size_t row = (size_t)(c0 + c) << LOG_M;
+            const size_t row = ((size_t)(c0 + c) << LOG_M) + brev((u32)g, S::LR1);
+            const double* tw = T.fmid + row;
+            u64* dst = out + base + row;
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) {
-                const size_t p = row + brev(S::R2 * g + e, LOG_M);
-                const double2 w = __ldg(T.fmid + p);
-                out[base + p] = (u64)__double_as_longlong(nttf::mulmod(y[e], w.x, w.y, qd));
+                const double w = __ldg(tw + brev_hi<LOG_M>(e));
+                dst[brev_hi<LOG_M>(e)] =
+                    (u64)__double_as_longlong(nttf::mulmod(y[e], w, __dmul_rn(w, qinv), qd));
             }
         }
         return;
@@ -167,7 +207,10 @@ k_fwd1(const void* __restrict__ in_, u64* __restrict__ out,
         if (kDigits) {
             const i64* in = (const i64*)in_ + ((size_t)blockIdx.z << (LOG_M + log_b));
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e) x[e] = lift_digit(in[c0 + c + ((size_t)(i0 + S::R2 * e) << log_b)], q, T.mu_hi);
+            for (int e = 0; e < S::R1; ++e) {
+                const i64 d = in[c0 + c + ((size_t)(i0 + S::R2 * e) << log_b)];
+                x[e] = small ? lift_small(d, q) : lift_digit(d, q, T.mu_hi);
+            }
         } else {
             const u64* in = (const u64*)in_ + base;
 #pragma unroll
@@ -198,12 +241,13 @@ k_fwd1(const void* __restrict__ in_, u64* __restrict__ out,
 // Forward pass 2 over units k_a: negacyclic B-point merged CT with
 // psi_2B = psi^A on {k_a + A j_lo}; output k_b = brev(r) stored at k_a + A k_b
 // (natural order). src may equal dst; values < 4q in, canonical out.
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(4))
 k_fwd2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
-       LimbMap lm, int limb_count, int log_a, int log_c) {
+       LimbMap lm, int limb_count, int log_a, int log_c_) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int limb = blockIdx.y;
     const NttTab& T = tabs[lm(limb)];
@@ -211,32 +255,41 @@ k_fwd2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
     const size_t base = ((size_t)blockIdx.z * limb_count + limb) << (LOG_M + log_a);
     const int b0 = blockIdx.x << log_c;
     const int c = tid & (C - 1);
-    if (LOG_M <= 8 && T.f64) {  // FP64 network: pass-1 doubles (below q in magnitude) in, canonical out
+    if (LOG_M <= 8 && T.f64) {  // FP64 network: pass-1 doubles (below 2 q in magnitude) in, canonical out
+        u64 raw[S::R1];
+        const bool act1 = tid < (C << S::LR2);
+        const int i0 = tid >> log_c;
+        if (act1) {  // before the table is staged: the two latencies overlap
+            const u64* in = src + base + b0 + c + ((size_t)i0 << log_a);
+            const size_t step = (size_t)S::R2 << log_a;
+#pragma unroll
+            for (int e = 0; e < S::R1; ++e) raw[e] = in[e * step];
+        }
         const double2* tab = stage_table_f64(sm + (S::M << log_c), T.fB, S::M);
         const double qd = T.qd, qinv = T.qinv;
         double* smd = reinterpret_cast<double*>(sm);
         auto twf = [&](int s, u32 blk) { return tab[(1u << s) + blk]; };
         __syncthreads();
-        if (tid < (C << S::LR2)) {
-            const int i0 = tid >> log_c;
+        if (act1) {
             double x[S::R1];
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e)
-                x[e] = __longlong_as_double((long long)src[base + ((size_t)(i0 + S::R2 * e) << log_a) + b0 + c]);
+            for (int e = 0; e < S::R1; ++e) x[e] = __longlong_as_double((long long)raw[e]);
             nttf::ct_stages<S::LR1>(x, 0, 0, twf, qd);
+            double* o = smd + (i0 << log_c) + c;
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e) smd[((i0 + S::R2 * e) << log_c) + c] = nttf::center(x[e], qd, qinv);
+            for (int e = 0; e < S::R1; ++e) o[(S::R2 * e) << log_c] = nttf::center(x[e], qd, qinv);
         }
         __syncthreads();
         if (tid < (C << S::LR1)) {
             const int g = tid >> log_c;
             double y[S::R2];
+            const double* o = smd + ((S::R2 * g) << log_c) + c;
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) y[e] = smd[((S::R2 * g + e) << log_c) + c];
+            for (int e = 0; e < S::R2; ++e) y[e] = o[e << log_c];
             nttf::ct_stages<S::LR2>(y, S::LR1, g, twf, qd);
+            u64* out = dst + base + b0 + c + ((size_t)brev((u32)g, S::LR1) << log_a);
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e)
-                dst[base + ((size_t)brev(S::R2 * g + e, LOG_M) << log_a) + b0 + c] = nttf::to_canonical(y[e], qd, qinv);
+            for (int e = 0; e < S::R2; ++e) out[(size_t)brev_hi<LOG_M>(e) << log_a] = nttf::to_canonical(y[e], qd, qinv);
         }
         return;
     }
@@ -283,17 +336,18 @@ k_fwd2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
 // Inverse pass 1 over units k_a: negacyclic B-point merged GS with psi_2B^-1
 // on the bit-reversed input {k_a + A brev(r)}, times the inverse twist
 // N^-1 psi^-((2k_a+1-A) j_lo), stored as row k_a (lazy, [0, 2q); limbs on the
-// FP64 network: doubles below 1.5 q in magnitude). in != out.
+// FP64 network: doubles below 3 q in magnitude). in != out.
 // With go.exps (sigma_k folded in), column j_lo of the row is stored at
 // position j_lo k mod B, so pass 2 reads the columns of each output column
 // together.
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(3))
 k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
        const NttTab* __restrict__ tabs, LimbMap lm, int limb_count,
-       int log_a, int log_c, GaloisOut go) {
+       int log_a, int log_c_, GaloisOut go) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int limb = blockIdx.y;
     const NttTab& T = tabs[lm(limb)];
@@ -301,6 +355,12 @@ k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
     const size_t base = ((size_t)blockIdx.z * limb_count + limb) << (LOG_M + log_a);
     const int b0 = blockIdx.x << log_c;
     const bool f64 = LOG_M <= 8 && T.f64;
+    u64 raw[S::R2];
+    if (tid < (C << S::LR1)) {  // before the table is staged: the two latencies overlap
+        const u64* src = in + base + b0 + (tid & (C - 1)) + ((size_t)brev((u32)(tid >> log_c), S::LR1) << log_a);
+#pragma unroll
+        for (int e = 0; e < S::R2; ++e) raw[e] = src[(size_t)brev_hi<LOG_M>(e) << log_a];
+    }
     u64* st = sm + (S::M << log_c);
     if (f64) stage_table_f64(st, T.fB_inv, S::M);
     else stage_table(st, T.psiB_inv, T.psiB_inv_q, S::M);
@@ -319,9 +379,7 @@ k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
         if (f64) {  // centred inputs, four GS stages (below 8 q), centred at the exchange
             double x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e)
-                x[e] = nttf::center(nttf::from_u52(in[base + ((size_t)brev(S::R2 * g + e, LOG_M) << log_a) + b0 + c]),
-                                    qd, qinv);
+            for (int e = 0; e < S::R2; ++e) x[e] = nttf::center(nttf::from_u52(raw[e]), qd, qinv);
             nttf::gs_stages<S::LR2>(x, 0, g, twf, qd);
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) {
@@ -331,7 +389,7 @@ k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
         } else {
             u64 x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) x[e] = in[base + ((size_t)brev(S::R2 * g + e, LOG_M) << log_a) + b0 + c];
+            for (int e = 0; e < S::R2; ++e) x[e] = raw[e];
             if (q < nttc::kLazyGsBound) nttc::gs_stages<S::LR2, true>(x, 0, g, tw, q);
             else nttc::gs_stages<S::LR2, false>(x, 0, g, tw, q);
 #pragma unroll
@@ -357,8 +415,8 @@ k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
             nttf::gs_stages<S::LR1>(y, S::LR2, 0, twf, qd);
 #pragma unroll
             for (int e = 0; e < S::R1; ++e) {
-                const double2 w = __ldg(T.fmidi + row + i0 + S::R2 * e);
-                v[e] = (u64)__double_as_longlong(nttf::mulmod(y[e], w.x, w.y, qd));
+                const double w = __ldg(T.fmidi + row + i0 + S::R2 * e);
+                v[e] = (u64)__double_as_longlong(nttf::mulmod(y[e], w, __dmul_rn(w, qinv), qd));
             }
         } else {
             u64 y[S::R1];
@@ -403,12 +461,13 @@ k_inv1(const u64* __restrict__ in, u64* __restrict__ out,
 // j_lo = p k^-1 mod B, and element i of it goes to coefficient
 // sigma_k(j_lo + B i) = p + B ((m + i k) mod 2A), m = floor((j_lo k mod 2N) / B),
 // negated past A rows; ib.b must then be null.
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(3))
 k_inv2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
-       LimbMap lm, int limb_count, int log_b, int log_c, InvBase ib, GaloisOut go) {
+       LimbMap lm, int limb_count, int log_b, int log_c_, InvBase ib, GaloisOut go) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int limb = blockIdx.y;
     const NttTab& T = tabs[lm(limb)];
@@ -417,6 +476,12 @@ k_inv2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
     const int c0 = blockIdx.x << log_c;
     const int c = tid & (C - 1);
     const bool f64 = LOG_M <= 8 && T.f64;
+    u64 raw[S::R2];
+    if (tid < (C << S::LR1)) {  // before the table is staged: the two latencies overlap
+        const u64* p = src + base + c0 + c + ((size_t)brev((u32)(tid >> log_c), S::LR1) << log_b);
+#pragma unroll
+        for (int e = 0; e < S::R2; ++e) raw[e] = p[(size_t)brev_hi<LOG_M>(e) << log_b];
+    }
     u64* st = sm + (S::M << log_c);
     if (f64) stage_table_f64(st, T.fA_inv, S::M);
     else stage_table(st, T.psiA_inv, T.psiA_inv_q, S::M);
@@ -432,20 +497,17 @@ k_inv2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
     __syncthreads();
     if (tid < (C << S::LR1)) {
         const int g = tid >> log_c;
-        if (f64) {  // pass-1 doubles (below 1.5 q) centred, four GS stages, centred at the exchange
+        if (f64) {  // pass-1 doubles (below 3 q) centred, four GS stages, centred at the exchange
             double x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e)
-                x[e] = nttf::center(
-                    __longlong_as_double((long long)src[base + c0 + c + ((size_t)brev(S::R2 * g + e, LOG_M) << log_b)]),
-                    qd, qinv);
+            for (int e = 0; e < S::R2; ++e) x[e] = nttf::center(__longlong_as_double((long long)raw[e]), qd, qinv);
             nttf::gs_stages<S::LR2>(x, 0, g, twf, qd);
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) smd[((S::R2 * g + e) << log_c) + c] = nttf::center(x[e], qd, qinv);
         } else {
             u64 x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) x[e] = src[base + c0 + c + ((size_t)brev(S::R2 * g + e, LOG_M) << log_b)];
+            for (int e = 0; e < S::R2; ++e) x[e] = raw[e];
             if (q < nttc::kLazyGsBound) nttc::gs_stages<S::LR2, true>(x, 0, g, tw, q);
             else nttc::gs_stages<S::LR2, false>(x, 0, g, tw, q);
 #pragma unroll
@@ -529,15 +591,22 @@ k_inv2(const u64* src, u64* dst, const NttTab* __restrict__ tabs,
 
 // Pass 2 of one limb of a column tile, sigma folded (k_inv2 with go.exps):
 // thread (i0, c) ends with v[e] = output row i0 + R2 e, column c0 + c.
-template <int LOG_M>
+template <int LOG_M, int LC>
 __device__ __forceinline__ void inv2_tile_folded(const u64* __restrict__ src, const NttTab& T, u64* sm, int log_b,
-                                                 int log_c, int c0, u32 poly, const GaloisOut& go, bool act,
+                                                 int log_c_, int c0, u32 poly, const GaloisOut& go, bool act,
                                                  u64 (&v)[Split<LOG_M>::R1]) {
     using S = Split<LOG_M>;
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int c = tid & (C - 1);
     const u64 q = T.q;
     const bool f64 = T.f64;
+    u64 raw[S::R2];
+    if (tid < (C << S::LR1)) {  // before the table is staged: the two latencies overlap
+        const u64* p = src + c0 + c + ((size_t)brev((u32)(tid >> log_c), S::LR1) << log_b);
+#pragma unroll
+        for (int e = 0; e < S::R2; ++e) raw[e] = p[(size_t)brev_hi<LOG_M>(e) << log_b];
+    }
     u64* st = sm + (S::M << log_c);
     if (f64) stage_table_f64(st, T.fA_inv, S::M);
     else stage_table(st, T.psiA_inv, T.psiA_inv_q, S::M);
@@ -556,17 +625,14 @@ __device__ __forceinline__ void inv2_tile_folded(const u64* __restrict__ src, co
         if (f64) {
             double x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e)
-                x[e] = nttf::center(
-                    __longlong_as_double((long long)src[c0 + c + ((size_t)brev(S::R2 * g + e, LOG_M) << log_b)]), qd,
-                    qinv);
+            for (int e = 0; e < S::R2; ++e) x[e] = nttf::center(__longlong_as_double((long long)raw[e]), qd, qinv);
             nttf::gs_stages<S::LR2>(x, 0, g, twf, qd);
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) smd[((S::R2 * g + e) << log_c) + c] = nttf::center(x[e], qd, qinv);
         } else {
             u64 x[S::R2];
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) x[e] = src[c0 + c + ((size_t)brev(S::R2 * g + e, LOG_M) << log_b)];
+            for (int e = 0; e < S::R2; ++e) x[e] = raw[e];
             if (q < nttc::kLazyGsBound) nttc::gs_stages<S::LR2, true>(x, 0, g, tw, q);
             else nttc::gs_stages<S::LR2, false>(x, 0, g, tw, q);
 #pragma unroll
@@ -625,12 +691,13 @@ __device__ __forceinline__ void inv2_tile_folded(const u64* __restrict__ src, co
 // One auxiliary limb (grid y: k, local limb q_limbs + k of the [polys][LK][N]
 // pass-1 output, table L_ctx + k) of a column tile, sigma folded, into
 // zp [polys][K][N] (canonical).
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(3))
 k_inv2_p(const u64* __restrict__ src, u64* __restrict__ zp, const NttTab* __restrict__ tabs, int q_limbs,
-         int L_ctx, int LK, int K, int log_b, int log_c, GaloisOut go) {
+         int L_ctx, int LK, int K, int log_b, int log_c_, GaloisOut go) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int c0 = blockIdx.x << log_c;
     const int k = blockIdx.y;
@@ -639,7 +706,7 @@ k_inv2_p(const u64* __restrict__ src, u64* __restrict__ zp, const NttTab* __rest
     const bool act = tid < (C << S::LR2);
     const int c = tid & (C - 1), i0 = tid >> log_c;
     u64 v[S::R1];
-    inv2_tile_folded<LOG_M>(src + (((size_t)poly * LK + q_limbs + k) << log_n), tabs[L_ctx + k], sm, log_b, log_c,
+    inv2_tile_folded<LOG_M, LC>(src + (((size_t)poly * LK + q_limbs + k) << log_n), tabs[L_ctx + k], sm, log_b, log_c,
                             c0, poly, go, act, v);
     if (act) {
         u64* o = zp + (((size_t)poly * K + k) << log_n);
@@ -670,13 +737,14 @@ __global__ void __launch_bounds__(256) k_pwords(const u64* __restrict__ zp, doub
 
 // One Q limb (grid x, fastest: the tile's words are reused from L2 by every
 // limb) of a column tile: pass 2, then ModDown into dst [polys][q_limbs][N].
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, min_ctas<LOG_M>(3))
 k_inv2_moddown(const u64* __restrict__ src, u64* __restrict__ dst, const double* __restrict__ words,
                const NttTab* __restrict__ tabs, const double* __restrict__ f64c, int q_limbs, int LK, int log_b,
-               int log_c, GaloisOut go) {
+               int log_c_, GaloisOut go) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const int limb = blockIdx.x;
     const int c0 = blockIdx.y << log_c;
@@ -685,7 +753,7 @@ k_inv2_moddown(const u64* __restrict__ src, u64* __restrict__ dst, const double*
     const bool act = tid < (C << S::LR2);
     const int c = tid & (C - 1), i0 = tid >> log_c;
     u64 v[S::R1];
-    inv2_tile_folded<LOG_M>(src + (((size_t)poly * LK + limb) << log_n), tabs[limb], sm, log_b, log_c, c0, poly, go,
+    inv2_tile_folded<LOG_M, LC>(src + (((size_t)poly * LK + limb) << log_n), tabs[limb], sm, log_b, log_c, c0, poly, go,
                             act, v);
     if (act) {
         double ci[12];
@@ -717,12 +785,13 @@ k_inv2_moddown(const u64* __restrict__ src, u64* __restrict__ dst, const double*
 //   mid  [n_ct][D][L][N]  pass-1 outputs of the digits (k_fwd1<_, true>)
 //   key  [D][2][L][N]     NTT-domain relinearization key
 //   base, acc [n_ct][2][L][N] (may alias)
-template <int LOG_M>
+template <int LOG_M, int LC>
 __global__ void __launch_bounds__(kMaxThreads, LOG_M <= 5 ? 3 : 2)
 k_fwd2_relin(const u64* __restrict__ mid, const u64* __restrict__ key, const u64* base, u64* acc,
-             const NttTab* __restrict__ tabs, int L, int D, int log_a, int log_c) {
+             const NttTab* __restrict__ tabs, int L, int D, int log_a, int log_c_) {
     using S = Split<LOG_M>;
     extern __shared__ u64 sm[];
+    const int log_c = LC >= 0 ? LC : log_c_;
     const int C = 1 << log_c, tid = threadIdx.x;
     const size_t ct = blockIdx.x;
     const int b0 = blockIdx.y << log_c;
@@ -739,35 +808,60 @@ k_fwd2_relin(const u64* __restrict__ mid, const u64* __restrict__ key, const u64
     double sb[S::R2], sa[S::R2];
 #pragma unroll
     for (int e = 0; e < S::R2; ++e) sb[e] = sa[e] = 0.0;
+    const bool act_a = tid < (C << S::LR2);
+    const size_t step = (size_t)S::R2 << log_a, digit = (size_t)L << log_n;
+    const u64* in = mid + ((ct * D * L + limb) << log_n) + b0 + c + ((size_t)g << log_a);
+    const u64* kb = key + ((size_t)limb << log_n) + b0 + c + ((size_t)brev((u32)g, S::LR1) << log_a);
+    // the next digit's words are loaded before this digit's key words are used, and the key
+    // words before the second half's stages, so neither latency stands alone (1024 outputs,
+    // 36 digits x 14 limbs of N = 2^15: 102 -> 74 ms)
+    u64 raw[S::R1];
+    if (act_a) {
+#pragma unroll
+        for (int e = 0; e < S::R1; ++e) raw[e] = in[e * step];
+    }
     __syncthreads();
     for (int j = 0; j < D; ++j) {
-        const size_t in_j = ((ct * D + j) * L + limb) << log_n;
-        if (tid < (C << S::LR2)) {
-            const int i0 = tid >> log_c;
+        if (act_a) {
             double x[S::R1];
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e)
-                x[e] = __longlong_as_double((long long)mid[in_j + ((size_t)(i0 + S::R2 * e) << log_a) + b0 + c]);
+            for (int e = 0; e < S::R1; ++e) x[e] = __longlong_as_double((long long)raw[e]);
             nttf::ct_stages<S::LR1>(x, 0, 0, twf, qd);
+            double* o = smd + (g << log_c) + c;
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e) smd[((i0 + S::R2 * e) << log_c) + c] = nttf::center(x[e], qd, qinv);
+            for (int e = 0; e < S::R1; ++e) o[(S::R2 * e) << log_c] = nttf::center(x[e], qd, qinv);
+            in += digit;
+            if (j + 1 < D) {
+#pragma unroll
+                for (int e = 0; e < S::R1; ++e) raw[e] = in[e * step];
+            }
         }
         __syncthreads();
         if (act_b) {
-            double y[S::R2];
+            constexpr bool kEarly = S::R2 <= 8;  // 16 key pairs beside 16 values would spill
+            u64 wb[S::R2], wa[S::R2];
+            auto key_words = [&](int e) {
+                wb[e] = __ldg(kb + ((size_t)brev_hi<LOG_M>(e) << log_a));
+                wa[e] = __ldg(kb + digit + ((size_t)brev_hi<LOG_M>(e) << log_a));
+            };
+            if (kEarly) {
 #pragma unroll
-            for (int e = 0; e < S::R2; ++e) y[e] = smd[((S::R2 * g + e) << log_c) + c];
+                for (int e = 0; e < S::R2; ++e) key_words(e);
+            }
+            double y[S::R2];
+            const double* o = smd + ((S::R2 * g) << log_c) + c;
+#pragma unroll
+            for (int e = 0; e < S::R2; ++e) y[e] = o[e << log_c];
             nttf::ct_stages<S::LR2>(y, S::LR1, g, twf, qd);
-            const u64* kb = key + ((((size_t)j * 2) * L + limb) << log_n) + b0 + c;
-            const u64* ka = kb + ((size_t)L << log_n);
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) {
-                const size_t pos = (size_t)brev(S::R2 * g + e, LOG_M) << log_a;
+                if (!kEarly) key_words(e);
                 const double v = nttf::center(y[e], qd, qinv);
-                const double wb = nttf::from_u52(__ldg(kb + pos)), wa = nttf::from_u52(__ldg(ka + pos));
-                sb[e] = __dadd_rn(sb[e], nttf::mulmod(v, wb, __dmul_rn(wb, qinv), qd));
-                sa[e] = __dadd_rn(sa[e], nttf::mulmod(v, wa, __dmul_rn(wa, qinv), qd));
+                const double db = nttf::from_u52(wb[e]), da = nttf::from_u52(wa[e]);
+                sb[e] = __dadd_rn(sb[e], nttf::mulmod(v, db, __dmul_rn(db, qinv), qd));
+                sa[e] = __dadd_rn(sa[e], nttf::mulmod(v, da, __dmul_rn(da, qinv), qd));
             }
+            kb += 2 * digit;
             if ((j & 7) == 7) {
 #pragma unroll
                 for (int e = 0; e < S::R2; ++e) {
@@ -808,40 +902,60 @@ int pick_log_c(int log_avail, int pref) {
     return pref >= 0 && pref <= mx ? pref : mx;
 }
 
+template <int LOG_M, int LC>
+void launch_pass_c(int which, const void* in, u64* out, const NttTab* tabs, LimbMap lm, u32 limbs, int log_other,
+                   int lc, dim3 grid, int threads, size_t smem, cudaStream_t st, const InvBase& ib,
+                   const GaloisOut& go, int digit_log) {
+    switch (which) {
+        case 0: k_fwd1<LOG_M, false, LC><<<grid, threads, smem, st>>>(in, out, tabs, lm, limbs, log_other, lc, 0); break;
+        case 1: k_fwd1<LOG_M, true, LC><<<grid, threads, smem, st>>>(in, out, tabs, lm, limbs, log_other, lc, digit_log); break;
+        case 2: k_fwd2<LOG_M, LC><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc); break;
+        case 3: k_inv1<LOG_M, LC><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc, go); break;
+        default: k_inv2<LOG_M, LC><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc, ib, go); break;
+    }
+}
+
+// The halves of the rings in use (2^6 .. 2^8 points) have their common column counts (8
+// and 16) as constants: exchange and stride addresses are then immediates.
 template <int LOG_M>
 int32_t launch_pass(int which, const void* in, u64* out, const NttTab* tabs, LimbMap lm, u32 limbs, u32 polys,
-                    int log_other, cudaStream_t st, const InvBase& ib, int lc_pref, const GaloisOut& go) {
+                    int log_other, cudaStream_t st, const InvBase& ib, int lc_pref, const GaloisOut& go,
+                    int digit_log) {
     const int lc = pick_log_c<LOG_M>(log_other, lc_pref);
     const int threads = Split<LOG_M>::RMAX << lc;
     const size_t smem = (sizeof(u64) << (LOG_M + lc)) + 2 * sizeof(u64) * (1u << LOG_M);
     dim3 grid(1u << (log_other - lc), limbs, polys);
-    switch (which) {
-        case 0: k_fwd1<LOG_M, false><<<grid, threads, smem, st>>>(in, out, tabs, lm, limbs, log_other, lc); break;
-        case 1: k_fwd1<LOG_M, true><<<grid, threads, smem, st>>>(in, out, tabs, lm, limbs, log_other, lc); break;
-        case 2: k_fwd2<LOG_M><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc); break;
-        case 3: k_inv1<LOG_M><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc, go); break;
-        default: k_inv2<LOG_M><<<grid, threads, smem, st>>>((const u64*)in, out, tabs, lm, limbs, log_other, lc, ib, go); break;
+    if constexpr (LOG_M >= 6 && LOG_M <= 8) {
+        if (lc == 4) {
+            launch_pass_c<LOG_M, 4>(which, in, out, tabs, lm, limbs, log_other, lc, grid, threads, smem, st, ib, go, digit_log);
+            return CKKS_OK;
+        }
+        if (lc == 3) {
+            launch_pass_c<LOG_M, 3>(which, in, out, tabs, lm, limbs, log_other, lc, grid, threads, smem, st, ib, go, digit_log);
+            return CKKS_OK;
+        }
     }
+    launch_pass_c<LOG_M, -1>(which, in, out, tabs, lm, limbs, log_other, lc, grid, threads, smem, st, ib, go, digit_log);
     return CKKS_OK;
 }
 
 int32_t pass(int which, int log_m, const void* in, u64* out, const NttTab* tabs, LimbMap lm, u32 limbs, u32 polys,
              int log_other, cudaStream_t st, const InvBase& ib = InvBase{}, int lc_pref = -1,
-             const GaloisOut& go = GaloisOut{}) {
+             const GaloisOut& go = GaloisOut{}, int digit_log = 0) {
     if (polys > 65535 || limbs > 65535) {  // grid y / z limits
         ckks_set_error("NTT: more than 65535 polynomials or limbs in one launch");
         return CKKS_ERR_BAD_ARG;
     }
     switch (log_m) {
-        case 1: return launch_pass<1>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 2: return launch_pass<2>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 3: return launch_pass<3>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 4: return launch_pass<4>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 5: return launch_pass<5>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 6: return launch_pass<6>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 7: return launch_pass<7>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 8: return launch_pass<8>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
-        case 9: return launch_pass<9>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go);
+        case 1: return launch_pass<1>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 2: return launch_pass<2>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 3: return launch_pass<3>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 4: return launch_pass<4>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 5: return launch_pass<5>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 6: return launch_pass<6>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 7: return launch_pass<7>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 8: return launch_pass<8>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
+        case 9: return launch_pass<9>(which, in, out, tabs, lm, limbs, polys, log_other, st, ib, lc_pref, go, digit_log);
         default: ckks_set_error("NTT: unsupported transform size"); return CKKS_ERR_BAD_ARG;
     }
 }
@@ -902,10 +1016,12 @@ int32_t ntt_inverse_base_launch(ckks_ctx* ctx, const u64* in, u64* out, u32 n_po
 }
 
 int32_t ntt_forward_digits_launch(ckks_ctx* ctx, const i64* digits, u64* out, u32 D, LimbMap lm, u32 limbs,
-                                  cudaStream_t st) {
+                                  cudaStream_t st, u32 base_log) {
     if (D == 0 || limbs == 0) return CKKS_OK;
     const int la = ctx->log_n1, lb = ctx->log_n2;
-    if (int32_t rc = pass(1, la, digits, out, ctx->d_tabs, lm, limbs, D, lb, st, InvBase{}, ctx->ntt_log_c[1])) return rc;
+    if (int32_t rc = pass(1, la, digits, out, ctx->d_tabs, lm, limbs, D, lb, st, InvBase{}, ctx->ntt_log_c[1],
+                          GaloisOut{}, (int)base_log))
+        return rc;
     if (int32_t rc = pass(2, lb, out, out, ctx->d_tabs, lm, limbs, D, la, st, InvBase{}, ctx->ntt_log_c[2])) return rc;
     CKKS_CUDA_TRY(cudaGetLastError());
     return CKKS_OK;
@@ -928,11 +1044,12 @@ bool ntt_relin_fused_supported(const ckks_ctx* ctx, u32 L) {
 // Bounded relinearization key sum of n_ct ciphertexts from their signed digits
 // [n_ct][D][N]: digit lift + forward pass 1 into mid, then k_fwd2_relin.
 int32_t ntt_relin_fused_launch(ckks_ctx* ctx, const i64* digits, u64* mid, const u64* key, const u64* base, u64* acc,
-                               u32 n_ct, u32 L, u32 D, cudaStream_t st) {
+                               u32 n_ct, u32 L, u32 D, cudaStream_t st, u32 base_log) {
     if (n_ct == 0) return CKKS_OK;
     const int la = ctx->log_n1, lb = ctx->log_n2;
     const LimbMap lm = LimbMap::range(0, L);
-    if (int32_t rc = pass(1, la, digits, mid, ctx->d_tabs, lm, L, n_ct * D, lb, st, InvBase{}, ctx->ntt_log_c[1]))
+    if (int32_t rc = pass(1, la, digits, mid, ctx->d_tabs, lm, L, n_ct * D, lb, st, InvBase{}, ctx->ntt_log_c[1],
+                          GaloisOut{}, (int)base_log))
         return rc;
     if (n_ct > 0x7FFFFFFFu || L > 65535) {
         ckks_set_error("relinearization: batch outside the launch limits");
@@ -943,8 +1060,9 @@ int32_t ntt_relin_fused_launch(ckks_ctx* ctx, const i64* digits, u64* mid, const
         const int lc = pick_log_c<LM>(la, kRelinLogC >= 0 ? kRelinLogC : ctx->ntt_log_c[2]);                  \
         const size_t smem = (sizeof(u64) << (LM + lc)) + 2 * sizeof(u64) * (1u << LM);                        \
         dim3 grid(n_ct, 1u << (la - lc), L);                                                                  \
-        k_fwd2_relin<LM><<<grid, Split<LM>::RMAX << lc, smem, st>>>(mid, key, base, acc, ctx->d_tabs, (int)L, \
-                                                                    (int)D, la, lc);                         \
+        constexpr int k4 = LM >= 6 ? 4 : -1, k3 = LM >= 6 ? 3 : -1;                                           \
+        auto* f = lc == 4 ? k_fwd2_relin<LM, k4> : lc == 3 ? k_fwd2_relin<LM, k3> : k_fwd2_relin<LM, -1>;     \
+        f<<<grid, Split<LM>::RMAX << lc, smem, st>>>(mid, key, base, acc, ctx->d_tabs, (int)L, (int)D, la, lc); \
     } while (0)
     switch (lb) {
         case 2: CKKS_RELIN_FUSED(2); break;
@@ -985,19 +1103,27 @@ int32_t ntt_inverse_moddown_launch(ckks_ctx* ctx, const u64* in, u64* mid, doubl
     const LimbMap lm = LimbMap::qp(ctx, q_limbs);
     if (int32_t rc = pass(3, lb, in, mid, ctx->d_tabs, lm, LK, polys, la, st, InvBase{}, ctx->ntt_log_c[3], go))
         return rc;
-#define CKKS_INV_MD(LM)                                                                                            \
-    do {                                                                                                           \
-        const int lc = pick_log_c<LM>(lb, ctx->ntt_log_c[4]);                                                      \
-        const int threads = Split<LM>::RMAX << lc;                                                                 \
-        const size_t smem = (sizeof(u64) << (LM + lc)) + 2 * sizeof(u64) * (1u << LM);                            \
-        k_inv2_p<LM><<<dim3(1u << (lb - lc), ctx->K, polys), threads, smem, st>>>(                                  \
-            mid, zp, ctx->d_tabs, (int)q_limbs, (int)ctx->L, (int)LK, (int)ctx->K, lb, lc, go);                    \
-        const dim3 gw((ctx->n + 255) / 256, polys);                                                                \
-        if (ctx->K == 1) k_pwords<1><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);              \
-        else if (ctx->K == 2) k_pwords<2><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);         \
-        else k_pwords<3><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);                          \
-        k_inv2_moddown<LM><<<dim3(q_limbs, 1u << (lb - lc), polys), threads, smem, st>>>(                          \
-            mid, out, words, ctx->d_tabs, ctx->mod_down.f64c, (int)q_limbs, (int)LK, lb, lc, go);                  \
+    auto run = [&](auto lm_c, auto lc_c) {
+        constexpr int LM = decltype(lm_c)::value, LC = decltype(lc_c)::value;
+        const int lc = pick_log_c<LM>(lb, ctx->ntt_log_c[4]);
+        const int threads = Split<LM>::RMAX << lc;
+        const size_t smem = (sizeof(u64) << (LM + lc)) + 2 * sizeof(u64) * (1u << LM);
+        k_inv2_p<LM, LC><<<dim3(1u << (lb - lc), ctx->K, polys), threads, smem, st>>>(
+            mid, zp, ctx->d_tabs, (int)q_limbs, (int)ctx->L, (int)LK, (int)ctx->K, lb, lc, go);
+        const dim3 gw((ctx->n + 255) / 256, polys);
+        if (ctx->K == 1) k_pwords<1><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);
+        else if (ctx->K == 2) k_pwords<2><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);
+        else k_pwords<3><<<gw, 256, 0, st>>>(zp, words, ctx->mod_down, (int)ctx->log_n);
+        k_inv2_moddown<LM, LC><<<dim3(q_limbs, 1u << (lb - lc), polys), threads, smem, st>>>(
+            mid, out, words, ctx->d_tabs, ctx->mod_down.f64c, (int)q_limbs, (int)LK, lb, lc, go);
+    };
+#define CKKS_INV_MD(LM)                                                                            \
+    do {                                                                                           \
+        constexpr std::integral_constant<int, LM> m{};                                             \
+        const int lc = pick_log_c<LM>(lb, ctx->ntt_log_c[4]);                                      \
+        if (LM >= 6 && lc == 4) run(m, std::integral_constant<int, LM >= 6 ? 4 : -1>{});           \
+        else if (LM >= 6 && lc == 3) run(m, std::integral_constant<int, LM >= 6 ? 3 : -1>{});      \
+        else run(m, std::integral_constant<int, -1>{});                                            \
     } while (0)
     switch (la) {
         case 1: CKKS_INV_MD(1); break;

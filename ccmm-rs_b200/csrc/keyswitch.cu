@@ -25,15 +25,20 @@ constexpr int kT = 256;
 // acc[1][l][k] =                                         sum_j Y[j][l][py(k)] * key[j][l][1][k]
 // py / pb: NTT-domain Galois source maps (k = 0: identity). blockIdx.z batches
 // ciphertexts: Y, base and acc advance by y_stride, b_stride, a_stride words.
+// perm_inv != 0: the key is stored permuted by its Galois element and a thread takes one
+// storage slot t, computing k = pi^-1(t) (perm_inv: the inverse element): the key's two
+// words a digit are then read in order and only Y's one word is gathered (N = 2^16,
+// 38 digits, 27 limbs: 341 -> 263 us; 162 us at the copy rate).
 __global__ void __launch_bounds__(kT) k_ks_mac(const u64* __restrict__ Y, const u64* __restrict__ key,
                                                const u64* __restrict__ base, const u64* __restrict__ pf,
                                                const u64* __restrict__ pf_q, u64* __restrict__ acc,
                                                const NttTab* __restrict__ tabs, LimbMap lm, int Lq, int LK, int D,
-                                               int log_n, u64 perm_y, u64 perm_b, u64 perm_key, size_t y_stride,
+                                               int log_n, u64 perm_y, u64 perm_b, u64 perm_inv, size_t y_stride,
                                                size_t b_stride, size_t a_stride) {
     const u32 n = 1u << log_n;
-    const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+    const u32 kk = blockIdx.x * blockDim.x + threadIdx.x;  // key slot
+    if (kk >= n) return;
+    const u32 k = perm_inv ? galois_src(kk, perm_inv, log_n) : kk;
     const int l = blockIdx.y;
     Y += blockIdx.z * y_stride;
     if (base) base += blockIdx.z * b_stride;
@@ -41,15 +46,29 @@ __global__ void __launch_bounds__(kT) k_ks_mac(const u64* __restrict__ Y, const 
     const NttTab& T = tabs[lm(l)];
     const u64 q = T.q, mu_hi = T.mu_hi, mu_lo = T.mu_lo;
     const u32 ky = perm_y ? galois_src(k, perm_y, log_n) : k;
-    const u32 kk = perm_key ? galois_src(k, perm_key, log_n) : k;  // key slot of k in permuted storage
     Acc128 ab{0, 0}, aa{0, 0};
     int since = 0;
-    for (int j = 0; j < D; ++j) {
-        u64 y = Y[(((size_t)j * LK + l) << log_n) + ky];
-        const u64* kp = key + ((((size_t)j * LK + l) * 2) << log_n);
-        ab.mac(y, kp[kk]);
-        aa.mac(y, kp[n + kk]);
-        if (++since == 15) {
+    const size_t y_step = (size_t)LK << log_n;
+    const u64 *yp = Y + ((size_t)l << log_n) + ky, *kp = key + (((size_t)l * 2) << log_n) + kk;
+    constexpr int kU = 5;  // digits in flight: the loads do not depend on each other
+    for (int j = 0; j < D; j += kU) {
+        u64 y[kU], kb[kU], ka[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (j + u < D) {
+                y[u] = __ldg(yp + u * y_step);
+                kb[u] = __ldcs(kp + 2 * u * y_step);
+                ka[u] = __ldcs(kp + 2 * u * y_step + n);
+            }
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (j + u < D) {
+                ab.mac(y[u], kb[u]);
+                aa.mac(y[u], ka[u]);
+            }
+        yp += kU * y_step;
+        kp += 2 * kU * y_step;
+        if ((since += kU) == 15) {
             ab.fold(q, mu_hi, mu_lo);
             aa.fold(q, mu_hi, mu_lo);
             since = 0;
@@ -334,6 +353,16 @@ int32_t relin_generate(ckks_ctx* ctx, ckks_ksk* key, const int8_t* secret, u64 s
 std::vector<int8_t> host_secret_automorphism(const int8_t* s, u32 n, u64 k) { return secret_automorphism(s, n, k); }
 
 // --------------------------------------------------------------- pipelines
+static u64 galois_inverse(u64 k, u32 n) {  // k^-1 mod 2N: the group has exponent N / 2
+    const u64 two_n = 2ull * n;
+    u64 r = 1, b = k % two_n;
+    for (u64 e = n - 1; e; e >>= 1) {
+        if (e & 1) r = r * b % two_n;
+        b = b * b % two_n;
+    }
+    return r;
+}
+
 int32_t ks_mac_launch(ckks_ctx* ctx, const u64* Y, const u64* key, const u64* base, u64* acc, u32 q_limbs, u32 D,
                       bool with_p, u64 perm_y, u64 perm_b, cudaStream_t st, u64 perm_key, u32 n_ct, size_t b_stride) {
     const u32 LK = with_p ? q_limbs + ctx->K : q_limbs;
@@ -345,7 +374,7 @@ int32_t ks_mac_launch(ckks_ctx* ctx, const u64* Y, const u64* key, const u64* ba
     dim3 g((ctx->n + kT - 1) / kT, LK, n_ct);
     k_ks_mac<<<g, kT, 0, st>>>(Y, key, base, with_p ? ctx->d_pmodq : nullptr, with_p ? ctx->d_pmodq + ctx->L : nullptr,
                                acc, ctx->d_tabs, lm, q_limbs, LK,
-                               D, ctx->log_n, perm_y, perm_b, perm_key, ((size_t)D * LK) << ctx->log_n, b_stride,
+                               D, ctx->log_n, perm_y, perm_b, perm_key ? galois_inverse(perm_key, ctx->n) : 0, ((size_t)D * LK) << ctx->log_n, b_stride,
                                ((size_t)2 * LK) << ctx->log_n);
     CKKS_CUDA_TRY(cudaGetLastError());
     return CKKS_OK;

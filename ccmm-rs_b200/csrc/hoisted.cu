@@ -19,6 +19,7 @@
 // loads) while the hoisted digit transforms of the group stay L2-resident
 // and are gathered through the permutation.
 #include "keyswitch.cuh"
+#include "ntt_core.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -310,6 +311,10 @@ __global__ void __launch_bounds__(kS * kLanes, 2) k_mac_tiled(const u64* __restr
 }
 
 }  // namespace
+
+namespace {
+#include "mac_f64.cuh"
+}
 
 // The tensor-core MAC runs on compute capability 10.0 devices (the library is
 // built for sm_100a only).
@@ -1181,6 +1186,13 @@ constexpr bool kFoldSigma = CKKS_FOLD_SIGMA != 0;
 #endif
 constexpr bool kFuseModDown = CKKS_FUSE_MODDOWN != 0;
 
+// (ciphertext, key) pairs of a group up to which the MAC runs on the FP64 pipe
+// (mac_f64.cuh). Measured at N=2^16, 24 + 3 limbs, D = 38: the tensor-core MAC takes
+// 21.3-21.5 ms for any number of pairs up to 16 x 32 (its items pad to 32 keys and 16
+// ciphertexts), the FP64 MAC 12.8 ms for 16 x 6 and 30.0 ms for 16 x 16 pairs, so the
+// lines cross near 180. It also needs no packed copy of the keys.
+constexpr size_t kF64MacPairs = 160;
+
 // Hoisted hybrid rotations of n_ct ciphertexts by n_keys Galois keys (bounded
 // or RNS-block gadget), out [n_ct][n_keys][2][Lq][N]. Ciphertexts are
 // processed in groups of up to 4 sharing each streamed key slice.
@@ -1197,12 +1209,17 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
     // (each key word read once per group), as far as device memory allows;
     // otherwise groups of 4 on the CUDA-core tiled MAC.
     bool use_tc = bounded && n >= (u32)tc::kTS && D < 4096 && ctx->tensor_cores && tc_enabled();
+    // few (ciphertext, key) pairs a group: the FP64 MAC (rule at kF64MacPairs)
+    const bool use_f64 = use_tc && D <= (u32)macf::kMaxDigits && n >= 16 &&
+                         (n_ct < kGroupMax ? n_ct : kGroupMax) * (size_t)n_keys <= kF64MacPairs;
     // the tensor-core MAC reads the keys' packed set (made on first use)
-    const PackedSet* pset = use_tc ? packed_set_get(ctx, keys, n_keys, st) : nullptr;
+    const PackedSet* pset = use_tc && !use_f64 ? packed_set_get(ctx, keys, n_keys, st) : nullptr;
     use_tc = pset != nullptr;
     ctx->last_mac_path = use_tc ? 1 : 0;
+    const bool with_base = use_tc || use_f64;  // the MAC adds P NTT(b) itself
     u32 G = n_ct >= 4 ? 4 : n_ct;
     if (use_tc) G = n_ct < pset->g_max ? n_ct : pset->g_max;
+    if (use_f64) G = n_ct < kGroupMax ? n_ct : kGroupMax;
     const int cap = 1024;
     const LimbMap lqp = LimbMap::qp(ctx, Lq);
     const size_t y_stride = (size_t)D * LK * n, d_stride = (size_t)D * n, f_stride = (size_t)n + 1,
@@ -1218,7 +1235,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
     // the group size was sized against the free memory when the key set was packed; if the
     // workspaces do not fit now, smaller groups are taken (same words, keys read more often)
     for (;;) {
-        if (!(rc = Y.alloc(G * y_stride, st)) && !(use_tc && (rc = Bh.alloc(G * b_stride, st))) &&
+        if (!(rc = Y.alloc(G * y_stride, st)) && !(with_base && (rc = Bh.alloc(G * b_stride, st))) &&
             !(rc = acc.alloc((size_t)G * n_keys * 2 * LK * n, st)) &&
             !(rc = Z.alloc((size_t)G * n_keys * 2 * LK * n, st)) &&
             !(rc = karr.alloc(3 * (size_t)n_keys + ctx->moduli.size(), st)) && !(rc = dig.alloc(G * d_stride, st)) &&
@@ -1234,7 +1251,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
     // (FP64 networks and ModDown); its P-CRT words
     // (and zp, the K auxiliary limbs of pass 2) need G * n_keys * 2 * N * (4 + K)
     // words, which the accumulators' buffer holds once pass 1 has read it
-    const bool fuse_md = use_tc && kFuseModDown && ntt_inverse_moddown_supported(ctx, Lq);
+    const bool fuse_md = with_base && kFuseModDown && ntt_inverse_moddown_supported(ctx, Lq);
     Workspace<u64> wsp;
     double* words = nullptr;
     u64* zp = nullptr;
@@ -1289,7 +1306,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
                                                ct_words)))
                 return rc;
             if ((rc = ntt_forward_digits_launch(ctx, dig.p, Y.p, D * gn, lqp, LK, st, k0->base_log))) return rc;
-            if (use_tc) {  // the tensor-core MAC takes P b as one more digit: NTT(b) on the Q limbs
+            if (with_base) {  // these MACs add P b in the NTT domain: NTT(b) on the Q limbs
                 CKKS_CUDA_TRY(cudaMemcpy2DAsync(Bh.p, b_stride * sizeof(u64), in0, ct_words * sizeof(u64),
                                                 b_stride * sizeof(u64), gn, cudaMemcpyDeviceToDevice, st));
                 if ((rc = ntt_forward_launch_map(ctx, Bh.p, Bh.p, gn, LimbMap::range(0, Lq), Lq, st))) return rc;
@@ -1324,6 +1341,14 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
                 Y.p, y_stride, Bh.p, b_stride, (int)Lq, pset->d, (int)pset->rg, d_keys, d_exps_inv, acc.p,
                 ctx->d_tabs, lqp, (int)gn,
                 (int)n_keys, (int)LK, (int)D, (int)ctx->log_n, exc.p, cnt.p, cap, d_psi, terr.p);
+        } else if (use_f64) {
+            macf::Args a{};
+            a.Y = Y.p, a.y_stride = y_stride, a.B = Bh.p, a.b_stride = b_stride;
+            a.keys = d_keys, a.exps_inv = d_exps_inv, a.acc = acc.p, a.tabs = ctx->d_tabs, a.lm = lqp;
+            a.n_ct = (int)gn, a.n_keys = (int)n_keys, a.Lq = (int)Lq, a.LK = (int)LK, a.D = (int)D;
+            a.log_n = (int)ctx->log_n, a.exc = exc.p, a.exc_count = cnt.p, a.cap = cap, a.psi = d_psi;
+            a.pf = ctx->d_pmodq, a.pf_q = ctx->d_pmodq + ctx->L;
+            if ((rc = macf::launch(ctx, a, st))) return rc;
         } else {
             const size_t smem = (size_t)(G >= 3 ? 4 : G) * D * kS * sizeof(u64);
             if (n >= (u32)kS && smem <= 200 * 1024) {
@@ -1361,8 +1386,8 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
         pt.begin(4);
         // inverse transform; the b components get P b of their ciphertext added on the
         // Q limbs (ModDown(x + P b) = ModDown(x) + b: the base term of the rotation)
-        InvBase ib;  // the tensor-core MAC already added P NTT(b) (base digit)
-        ib.b = use_tc ? nullptr : ct_in + (size_t)c0 * ct_words;
+        InvBase ib;  // the tensor-core and FP64 MACs already added P NTT(b)
+        ib.b = with_base ? nullptr : ct_in + (size_t)c0 * ct_words;
         ib.b_stride = ct_words;
         ib.n_keys = n_keys;
         ib.q_limbs = Lq;
@@ -1372,7 +1397,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
         // streams without a gather); the CUDA-core path adds P b in the inverse
         // transform and applies sigma_g in ModDown
         GaloisOut go;
-        if (use_tc && kFoldSigma) {
+        if (with_base && kFoldSigma) {
             go.exps = d_exps;
             go.exps_inv = d_exps_inv;
             go.n_keys = n_keys;
@@ -1415,7 +1440,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
             CKKS_CUDA_TRY(cudaStreamSynchronize(st));
         }
         if (h_err) {
-            ckks_set_error("key-switch MAC: a tensor-core pipeline wait timed out");
+            ckks_set_error("key-switch MAC: a pipeline wait timed out");
             return CKKS_ERR_TIMEOUT;
         }
         for (u32 c = 0; c < gn; ++c)

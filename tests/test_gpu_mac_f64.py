@@ -1,0 +1,61 @@
+"""GPU tests of the key-switch MAC on the FP64 pipe (csrc/mac_f64.cuh):
+equal to the CUDA-core MAC word for word, and to the oracle on sampled pairs."""
+import numpy as np
+import pytest
+
+import ckks_b200 as cb
+from ckks_b200.params import chain
+
+pytestmark = pytest.mark.gpu
+
+
+def setup(log_n, q_bits, p_bits, n_ct, steps, base_log, seed, plant=False):
+    q, p = chain(1 << log_n, q_bits, p_bits)
+    ctx = cb.Context(log_n, q, p)
+    n = ctx.n
+    rng = np.random.default_rng(seed)
+    s = rng.integers(-1, 2, n).astype(np.int8)
+    ks = [ctx.rotation_exponent_left(r) for r in steps]
+    keys = [cb.KeySwitchKey.hybrid_generate(ctx, len(q), base_log, k, s, seed=seed + i) for i, k in enumerate(ks)]
+    cts = np.stack([np.stack([rng.integers(0, m, (2, n), dtype=np.uint64) for m in q], axis=1) for _ in range(n_ct)])
+    if plant:  # a parts whose balanced digits contain -B/2: the carry corrections
+        Q = int(np.prod([int(m) for m in q], dtype=object))
+        for c in range(0, n, 5):
+            v = (Q - (1 << (base_log - 1)) * (1 + (c % 3) * (1 << base_log))) % Q
+            cts[0, 1, :, c] = [v % m for m in q]
+    return q, p, ctx, ks, keys, cts
+
+
+# pieces of two and of three (60-bit limbs in Q), one key (two components a thread), one
+# ciphertext, partial ciphertext and key groups, several key chunks, the smallest ring,
+# digit counts odd and beyond two folds (base 2^8: 38 digits), 160 pairs exactly
+@pytest.mark.parametrize("log_n,q_bits,p_bits,n_ct,n_keys,base_log,plant", [
+    (4, (30,) * 3, (31,), 5, 4, 8, False),
+    (10, (50,) * 3, (60,), 1, 1, 32, True),
+    (10, (50,) * 6, (60, 60), 16, 10, 8, False),
+    (10, (60, 40, 40), (60,), 7, 3, 20, True),
+    (11, (50,) * 4, (60,) * 3, 13, 9, 32, True),
+    (10, (55,) * 2, (61,), 2, 17, 32, False),
+    (12, (50,) * 9, (60,), 3, 6, 8, False),
+])
+def test_f64_mac_equals_cuda_core_mac(oracle, cuda, log_n, q_bits, p_bits, n_ct, n_keys, base_log, plant):
+    q, p, ctx, ks, keys, cts = setup(log_n, q_bits, p_bits, n_ct, range(1, n_keys + 1), base_log, 31 + n_ct, plant)
+    d = cb.as_u64_tensor(cts)
+    got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d))
+    assert ctx.last_mac_path == "cuda_cores"
+    ctx.tensor_cores = False
+    assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d)))
+    for c, g in {(0, 0), (n_ct - 1, n_keys - 1)}:
+        want = oracle.hybrid_rotate(q, p, keys[g].download(), ks[g], base_log, cts[c])
+        assert np.array_equal(got[c, g], want), (c, g)
+
+
+def test_tensor_core_mac_corrections_in_a_full_group(cuda):
+    """16 x 18 pairs stay on the tensor-core MAC: its carry corrections against the CUDA-core MAC's."""
+    q, p, ctx, ks, keys, cts = setup(12, (50,) * 4, (60,), 16, range(1, 19), 32, 91, plant=True)
+    d = cb.as_u64_tensor(cts)
+    got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d))
+    assert ctx.last_mac_path == "tensor_cores"
+    ctx.tensor_cores = False
+    assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d)))
+

@@ -1341,11 +1341,12 @@ def bench_park_gpu(args, world, rank, local):
     torch.cuda.synchronize()
     e2e_s = e0.elapsed_time(e1) / 1000.0 / args.steps
     e2e_equal = bool(torch.equal(Ch, C.cpu()))
-    # the dominant kernel k_park_tc runs nb^2 n^3 unsigned 8-bit multiply-adds (nb = 5 bytes
-    # per residue of the 35-bit modulus) on the tensor cores; INT8 dense is twice the bf16
-    # dense rate on B200, so the peak is twice the measured bf16 burst figure
-    nb = ((q - 1).bit_length() + 7) // 8
-    ops = 2.0 * nb * nb * float(n) ** 3
+    # the dominant kernel k_rns_gemm runs one n^3 product of unsigned bytes per modulus of the
+    # residue system (11 for the 35-bit modulus at n = 4096: product above 2 n (q - 1)^2) on the
+    # tensor cores; INT8 dense is twice the bf16 dense rate on B200, so the peak is twice the
+    # measured bf16 burst figure. The timed span holds the combining pass as well.
+    n_mod = park_moduli(n, q)
+    ops = 2.0 * n_mod * float(n) ** 3
     bf16, bf16_kind = bf16_peak()
     i8_peak = 2.0 * bf16 if bf16 else None
     achieved = ops / (gemm / 1000.0) / 1e12
@@ -1356,11 +1357,10 @@ def bench_park_gpu(args, world, rank, local):
             "config": park_config(n),
             "roofline": {"bound": "tensor", "achieved": achieved, "unit": "TOP/s (INT8)", "peak": i8_peak,
                          "frac": achieved / i8_peak if i8_peak else None,
-                         # DRAM bytes of one launch at n = 2048 (read 127.0 MB, write 23.4 MB: the
-                         # packed operands once and the product), scaled by n^2 like those arrays
-                         "traffic": (127.0e6 + 23.4e6) * (n / 2048.0) ** 2,
-                         "traffic_source": "ncu capture of the n=2048 launch, scaled by (n/2048)^2",
-                         "kernel": "k_park_tc (INT8 tcgen05 products of byte planes, %d x %d planes)" % (nb, nb),
+                         # packed operands and residues of the product once each, and the product
+                         "traffic": (4.0 * n_mod + 8.0) * n * n,
+                         "traffic_source": "algorithmic bytes of the product and combining passes",
+                         "kernel": "k_rns_gemm + k_rns_combine (INT8 tcgen05 products of %d residues)" % n_mod,
                          "kernel_ms": gemm, "rest_of_step_ms": (ms_max / args.steps) - gemm,
                          "peak_source": "2 x bf16 dense (%s %s)" % (bf16_kind, bf16),
                          "ops_per_launch": ops},
@@ -1372,6 +1372,16 @@ def bench_park_gpu(args, world, rank, local):
             "parity": {"words_compared": len(rows) * n, "mismatches": mism,
                        "what": "three full output rows against the oracle's Reference backend"},
             "gpu_launches": 3 * args.steps, "clocks": clk}
+
+
+def park_moduli(n, q):
+    """Moduli of the residue-system product (csrc/park.cu, rns::moduli_for)."""
+    need, have = 1.05 + np.log2(n) + 2.0 * np.log2(q - 1), 0.0
+    for i, m in enumerate((256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193)):
+        have += np.log2(m)
+        if have > need:
+            return i + 1
+    raise ValueError("modulus too wide for the residue system")
 
 
 def park_metric(n):

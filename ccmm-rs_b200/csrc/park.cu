@@ -23,11 +23,27 @@
 // four epilogue warps (plane combine, one reduction per output); the two TMEM
 // accumulator sets let a tile's epilogue overlap the next tile's MMAs.
 //
+// Residue system (tensor cores, moduli of 4 bytes or more below 2^62). The byte planes
+// cost nb^2 products; a product modulo small coprime m_i <= 256 costs one, and the exact
+// integer sum X < inner (q - 1)^2 is determined by its residues once prod m_i = M > 2 X:
+// 11 products instead of 25 for a 35-bit q at inner = 4096, 17 instead of 64 for 60 bits.
+// With A_i = lhs mod m_i, B_i = rhs (M / m_i)^-1 mod m_i (bytes), w_i = A_i B_i mod m_i:
+//   X = sum_i w_i (M / m_i) - k M,   k = floor(sum_i w_i / m_i)  (X / M < 1/2),
+// so out = sum_i w_i (M / m_i mod q) - k (M mod q) mod q, with k from 2^27-scaled integer
+// reciprocals (each below the true one by under 2^-27: the sum is off by under 2^-14).
+// Packing takes two byte dot products an element and modulus; the GEMM is the persistent
+// kernel below with N = 256 and one accumulator, storing w_i as bytes; one kernel combines
+// the n_mod bytes of an output. n = 4096, 35-bit q: packing 0.17 ms, GEMM 0.54 ms (2.80 POP/s,
+// 88 % of twice the bf16 rate: the tensor pipe bounds it), combining 0.12 ms; the byte planes
+// took 0.26 and 1.24 ms.
+//
 // CUDA cores. A CTA computes a 64 x 64 block of outputs with 256 threads (4 x 4
 // outputs each, strided by 16 so a warp's loads of a staged tile row are
 // consecutive), staging 16-deep slices of both operands in shared memory; each
 // dot product is summed exactly in 192 bits (any u64 inputs, up to 2^64 terms)
 // and reduced once.
+#include <cmath>
+
 #include "context.cuh"
 #include "kernels.cuh"
 #include "tcgen05.cuh"
@@ -409,13 +425,10 @@ int32_t timing_events(int dev) {
     return CKKS_OK;
 }
 
-template <int NB>
-int32_t launch(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 cols, u64 q, cudaStream_t st) {
-    constexpr int kCt = cols_per_tile(NB), kRows = NB * kCt, kChunk = blocks_per_launch(NB);
-    const int n_mt = (int)((rows + 127) / 128), n_nt = (int)((cols + kCt - 1) / kCt), n_kb = (int)((inner + 31) / 32);
-    int dev = 0, n_sm = 0;
-    CKKS_CUDA_TRY(cudaGetDevice(&dev));
-    CKKS_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+// Runs body(err, packed): `err` a zeroed device word for the role of a timed-out wait,
+// packed() called between the packing and the product; then waits and reports.
+template <typename F>
+int32_t timed(int dev, cudaStream_t st, F&& body) {
     {  // keep the freed packed operands cached in the device pool between calls
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
@@ -423,36 +436,18 @@ int32_t launch(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u3
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
         }
     }
-    Workspace<uint8_t> ap, bp;
     Workspace<int> err;
     int32_t rc;
-    if ((rc = ap.alloc((size_t)n_mt * n_kb * NB * kATile, st)) ||
-        (rc = bp.alloc((size_t)n_nt * n_kb * NB * kRows * 32, st)) || (rc = err.alloc(1, st)))
-        return rc;
+    if ((rc = err.alloc(1, st))) return rc;
     CKKS_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(int), st));
     if ((rc = timing_events(dev))) return rc;
     t_timing.pack_ms = t_timing.gemm_ms = -1.f;
     CKKS_CUDA_TRY(cudaEventRecord(t_timing.ev[0], st));
-    auto grid_of = [&](size_t threads) {
-        const size_t g = (threads + 255) / 256, cap = (size_t)n_sm * 16;
-        return (int)(g < cap ? g : cap);
+    auto packed = [&]() -> int32_t {
+        CKKS_CUDA_TRY(cudaEventRecord(t_timing.ev[1], st));
+        return CKKS_OK;
     };
-    k_pack_a<<<grid_of((size_t)n_mt * 128 * 2 * n_kb), 256, 0, st>>>(lhs, ap.p, (int)rows, (int)inner, q, NB, n_mt,
-                                                                       n_kb);
-    CKKS_CUDA_TRY(cudaGetLastError());
-    const u64 f256q = (q > 256 && q <= (1ull << 63)) ? (u64)(((u128)256 << 64) / q) : 0;
-    k_pack_b<<<grid_of((size_t)n_nt * kCt * 2 * n_kb), 256, 0, st>>>(rhs, bp.p, (int)inner, (int)cols, q, NB, kCt,
-                                                                      n_nt, n_kb, f256q);
-    CKKS_CUDA_TRY(cudaGetLastError());
-    CKKS_CUDA_TRY(cudaFuncSetAttribute(k_park_tc<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-    const int n_tiles = n_mt * n_nt, grid = n_tiles < n_sm ? n_tiles : n_sm;
-    CKKS_CUDA_TRY(cudaEventRecord(t_timing.ev[1], st));
-    for (int kb0 = 0; kb0 < n_kb; kb0 += kChunk) {
-        const int kb1 = kb0 + kChunk < n_kb ? kb0 + kChunk : n_kb;
-        k_park_tc<NB><<<grid, kThreads, kSmemBytes, st>>>(ap.p, bp.p, out, (int)rows, (int)cols, q, n_mt, n_nt, n_kb,
-                                                          kb0, kb1, kb0 > 0 ? 1 : 0, err.p);
-        CKKS_CUDA_TRY(cudaGetLastError());
-    }
+    if ((rc = body(err.p, packed))) return rc;
     CKKS_CUDA_TRY(cudaEventRecord(t_timing.ev[2], st));
     int h_err = 0;
     CKKS_CUDA_TRY(cudaMemcpyAsync(&h_err, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -465,6 +460,43 @@ int32_t launch(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u3
         return CKKS_ERR_TIMEOUT;
     }
     return CKKS_OK;
+}
+
+template <int NB>
+int32_t launch(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 cols, u64 q, cudaStream_t st) {
+    constexpr int kCt = cols_per_tile(NB), kRows = NB * kCt, kChunk = blocks_per_launch(NB);
+    const int n_mt = (int)((rows + 127) / 128), n_nt = (int)((cols + kCt - 1) / kCt), n_kb = (int)((inner + 31) / 32);
+    int dev = 0, n_sm = 0;
+    CKKS_CUDA_TRY(cudaGetDevice(&dev));
+    CKKS_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    return timed(dev, st, [&](int* err, auto packed) -> int32_t {
+        Workspace<uint8_t> ap, bp;
+        int32_t rc;
+        if ((rc = ap.alloc((size_t)n_mt * n_kb * NB * kATile, st)) ||
+            (rc = bp.alloc((size_t)n_nt * n_kb * NB * kRows * 32, st)))
+            return rc;
+        auto grid_of = [&](size_t threads) {
+            const size_t g = (threads + 255) / 256, cap = (size_t)n_sm * 16;
+            return (int)(g < cap ? g : cap);
+        };
+        k_pack_a<<<grid_of((size_t)n_mt * 128 * 2 * n_kb), 256, 0, st>>>(lhs, ap.p, (int)rows, (int)inner, q, NB, n_mt,
+                                                                           n_kb);
+        CKKS_CUDA_TRY(cudaGetLastError());
+        const u64 f256q = (q > 256 && q <= (1ull << 63)) ? (u64)(((u128)256 << 64) / q) : 0;
+        k_pack_b<<<grid_of((size_t)n_nt * kCt * 2 * n_kb), 256, 0, st>>>(rhs, bp.p, (int)inner, (int)cols, q, NB, kCt,
+                                                                          n_nt, n_kb, f256q);
+        CKKS_CUDA_TRY(cudaGetLastError());
+        CKKS_CUDA_TRY(cudaFuncSetAttribute(k_park_tc<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        const int n_tiles = n_mt * n_nt, grid = n_tiles < n_sm ? n_tiles : n_sm;
+        if ((rc = packed())) return rc;
+        for (int kb0 = 0; kb0 < n_kb; kb0 += kChunk) {
+            const int kb1 = kb0 + kChunk < n_kb ? kb0 + kChunk : n_kb;
+            k_park_tc<NB><<<grid, kThreads, kSmemBytes, st>>>(ap.p, bp.p, out, (int)rows, (int)cols, q, n_mt, n_nt,
+                                                              n_kb, kb0, kb1, kb0 > 0 ? 1 : 0, err);
+            CKKS_CUDA_TRY(cudaGetLastError());
+        }
+        return CKKS_OK;
+    });
 }
 
 // the tensor-core form covers every modulus; tile counts stay within int
@@ -488,6 +520,399 @@ int32_t run(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 c
 }
 
 }  // namespace ptc
+
+// ------------------------------------------------------- residue number system
+namespace rns {
+
+using namespace tcg;
+
+constexpr int kMaxMod = 20;
+// pairwise coprime, descending: 256 = 2^8, 255 = 3 5 17, 253 = 11 23, 247 = 13 19, 217 = 7 31, primes
+constexpr int kModuli[kMaxMod] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227,
+                                  223, 217, 211, 199, 197, 193, 191, 181, 179, 173};
+constexpr int kMaxInner = 33024;  // 33024 * 255^2 < 2^31
+constexpr int kN = 256;           // output columns per tile
+constexpr u32 kATile = 128 * 32, kBTile = kN * 32;
+constexpr int kSteps = 4, kStages = 4;  // 32-byte inner steps per stage, stages
+constexpr u32 kOffB = kSteps * kATile, kStageBytes = kOffB + kSteps * kBTile;
+constexpr u32 kSmemBytes = kStages * kStageBytes;  // 192 KB
+constexpr u32 kIdesc = idesc_i8(128, kN, false);
+constexpr int kEpiWarps = 4, kProdWarp = 4, kMmaWarp = 5, kThreads = 32 * 6, kEpi = 128, kBarEpi = 1;
+
+struct Mod {
+    u32 m, mu_small, mu;      // modulus; ceil(2^32 / m) (exact quotients below 2^24), floor(2^32 / m)
+    u32 a_lo, a_hi;           // bytes 2^(8j) mod m, j = 0..3, 4..7
+    u32 b_lo, b_hi;           // bytes 2^(8j) (M / m)^-1 mod m
+    u32 recip;                // floor(2^27 / m)
+    u32 mq_lo, mq_hi;         // M / m mod q
+};
+struct Params {
+    int n;
+    Mod m[kMaxMod];
+    u64 q, mu, r32, r32q;     // floor((2^64 - 1) / q), 2^32 mod q and its Shoup companion
+    u32 nm_lo, nm_hi;         // q - (M mod q)
+};
+
+// x mod m from the byte dot product with 2^(8j) mod m: below 2^19 + 2^19, exact quotient
+__device__ __forceinline__ u32 residue(u32 lo, u32 hi, u32 r_lo, u32 r_hi, const Mod& md) {
+    const u32 s = __dp4a(lo, r_lo, __dp4a(hi, r_hi, 0u));
+    return s - __umulhi(s, md.mu_small) * md.m;
+}
+
+// Both operands: per modulus 32-byte inner steps in the K-major core-matrix order.
+// A' [n][n_mt][n_kb][128 x 32]: one thread per (row, 16-deep run); B' [n][n_nt][n_kb][256 x 32]:
+// one thread per (column, 16-deep run). Threads [0, a_total) take A. Neighbouring threads take
+// neighbouring rows (columns), so a warp stores whole 128-byte core matrices.
+__global__ void __launch_bounds__(256) k_rns_pack(const u64* __restrict__ A, const u64* __restrict__ B,
+                                                  uint8_t* __restrict__ Ap, uint8_t* __restrict__ Bp, int rows,
+                                                  int inner, int cols, int n_mt, int n_nt, int n_kb, bool vec_a,
+                                                  const __grid_constant__ Params P) {
+    const size_t runs = (size_t)2 * n_kb, a_total = (size_t)n_mt * 128 * runs, b_total = (size_t)n_nt * kN * runs;
+    const size_t a_plane = (size_t)n_mt * n_kb * kATile, b_plane = (size_t)n_nt * n_kb * kBTile;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < a_total + b_total;
+         t += (size_t)gridDim.x * blockDim.x) {
+        const bool is_a = t < a_total;
+        u64 v[16];
+        uint8_t* dst;
+        if (is_a) {
+            const int rpad = n_mt * 128, row = (int)(t % rpad), h = (int)(t / rpad);
+            const u64* src = A + (size_t)row * inner + 16 * h;
+            if (vec_a && row < rows && 16 * h + 16 <= inner) {
+#pragma unroll
+                for (int e = 0; e < 16; e += 2) {
+                    const ulonglong2 x = __ldg((const ulonglong2*)(src + e));
+                    v[e] = x.x, v[e + 1] = x.y;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] = (row < rows && 16 * h + e < inner) ? src[e] : 0;
+            }
+            dst = Ap + ((size_t)(row >> 7) * n_kb + (h >> 1)) * kATile + ptc::core_off(row & 127, h & 1);
+        } else {
+            const size_t u = t - a_total;
+            const int cpad = n_nt * kN, c = (int)(u % cpad), h = (int)(u / cpad);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const int k = 16 * h + e;
+                v[e] = (c < cols && k < inner) ? B[(size_t)k * cols + c] : 0;
+            }
+            dst = Bp + ((size_t)(c / kN) * n_kb + (h >> 1)) * kBTile + ptc::core_off(c % kN, h & 1);
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = v[e] < P.q ? v[e] : v[e] % P.q;
+        const size_t plane = is_a ? a_plane : b_plane;
+        for (int i = 0; i < P.n; ++i, dst += plane) {
+            const Mod& md = P.m[i];
+            const u32 r_lo = is_a ? md.a_lo : md.b_lo, r_hi = is_a ? md.a_hi : md.b_hi;
+            u32 w[4];
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                w[g] = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    w[g] |= residue((u32)v[4 * g + e], (u32)(v[4 * g + e] >> 32), r_lo, r_hi, md) << (8 * e);
+            }
+            *(uint4*)dst = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+// Every (modulus, row tile, column tile): w_i = A_i B_i mod m_i as bytes W [n][128 n_mt][256 n_nt].
+// Roles and waits as k_park_tc; row tiles vary fastest, then column tiles, then moduli.
+__global__ void __launch_bounds__(kThreads, 1)
+    k_rns_gemm(const uint8_t* __restrict__ Ap, const uint8_t* __restrict__ Bp, uint8_t* __restrict__ W, int n_mt,
+               int n_nt, int n_kb, const __grid_constant__ Params P, int* __restrict__ err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ u32 s_tmem;
+    __shared__ int s_abort;
+    __shared__ __align__(8) uint64_t s_full[kStages], s_empty[kStages], s_tfull[2], s_tfree[2];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int per_mod = n_mt * n_nt, n_tiles = per_mod * P.n;
+    const int my_tiles = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (tid == 0) {
+        s_abort = 0;
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(smem_u32(&s_full[i]), 1);
+            mbar_init(smem_u32(&s_empty[i]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&s_tfull[i]), 1);
+            mbar_init(smem_u32(&s_tfree[i]), 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(512u));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const u32 tmem = s_tmem, sbase = smem_u32(smem);
+
+    if (warp == kProdWarp) {
+        // ------------------------------------------------------------ producer
+        if (lane == 0) {
+            int g = 0;
+            bool bad = false;
+            for (int lt = 0; lt < my_tiles && !bad; ++lt) {
+                const int t = (int)blockIdx.x + lt * (int)gridDim.x, i = t / per_mod, x = t - i * per_mod;
+                const int nt = x / n_mt, mt = x - nt * n_mt;
+                const uint8_t* a = Ap + ((size_t)i * n_mt + mt) * n_kb * kATile;
+                const uint8_t* b = Bp + ((size_t)i * n_nt + nt) * n_kb * kBTile;
+                for (int s = 0; s < n_kb; s += kSteps, ++g) {
+                    const int st = g % kStages;
+                    const u32 n = (u32)(n_kb - s < kSteps ? n_kb - s : kSteps);
+                    if ((g >= kStages && !wait_parity(smem_u32(&s_empty[st]), (u32)(((g / kStages) - 1) & 1))) ||
+                        s_abort) {
+                        atomicExch(err, 1);
+                        s_abort = 1;
+                        bad = true;
+                        break;
+                    }
+                    const u32 bar = smem_u32(&s_full[st]), dst = sbase + (u32)st * kStageBytes;
+                    expect_tx(bar, n * (kATile + kBTile));
+                    bulk_g2s(dst, a + (size_t)s * kATile, n * kATile, bar);
+                    bulk_g2s(dst + kOffB, b + (size_t)s * kBTile, n * kBTile, bar);
+                }
+            }
+            // every copy issued has landed before the CTA can leave (bounded)
+            for (int x = g - kStages < 0 ? 0 : g - kStages; x < g; ++x)
+                wait_parity(smem_u32(&s_full[x % kStages]), (u32)((x / kStages) & 1));
+        }
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        // ------------------------------------------------------------ MMA issue
+        if (lane == 0) {
+            int g = 0, last = -1;
+            bool bad = false;
+            for (int lt = 0; lt < my_tiles && !bad; ++lt) {
+                const int buf = lt & 1;
+                if (lt >= 2 && !wait_parity(smem_u32(&s_tfree[buf]), (u32)(((lt >> 1) - 1) & 1))) {
+                    atomicExch(err, 3);
+                    s_abort = 1;
+                    break;
+                }
+                fence_after();
+                for (int s = 0; s < n_kb; s += kSteps, ++g) {
+                    const int st = g % kStages;
+                    const int n = n_kb - s < kSteps ? n_kb - s : kSteps;
+                    if (!wait_parity(smem_u32(&s_full[st]), (u32)((g / kStages) & 1)) || s_abort) {
+                        atomicExch(err, 2);
+                        s_abort = 1;
+                        bad = true;
+                        break;
+                    }
+                    fence_after();
+                    const u32 a_addr = sbase + (u32)st * kStageBytes, b_addr = a_addr + kOffB;
+#pragma unroll
+                    for (int u = 0; u < kSteps; ++u)
+                        if (u < n)
+                            mma_i8(tmem + (u32)buf * 256u, sdesc(a_addr + (u32)u * kATile, ptc::kLbo, ptc::kSbo),
+                                   sdesc(b_addr + (u32)u * kBTile, ptc::kLbo, ptc::kSbo), kIdesc, (s + u) > 0 ? 1u : 0u);
+                    commit(smem_u32(&s_empty[st]));
+                    last = g;
+                }
+                if (!bad) commit(smem_u32(&s_tfull[buf]));
+            }
+            // the last commit covers every MMA issued
+            if (last >= 0) wait_parity(smem_u32(&s_empty[last % kStages]), (u32)((last / kStages) & 1));
+        }
+        __syncwarp();
+    } else if (warp < kEpiWarps) {
+        // ------------------------------------------------------------- epilogue
+        for (int lt = 0; lt < my_tiles; ++lt) {
+            const int buf = lt & 1;
+            const int t = (int)blockIdx.x + lt * (int)gridDim.x, i = t / per_mod, x = t - i * per_mod;
+            const int nt = x / n_mt, mt = x - nt * n_mt;
+            const bool bad = !wait_parity(smem_u32(&s_tfull[buf]), (u32)((lt >> 1) & 1));
+            if (group_any(kBarEpi, kEpi, bad || s_abort)) {
+                if (tid == 0) {
+                    atomicExch(err, 4);
+                    s_abort = 1;
+                }
+                break;
+            }
+            fence_after();
+            const u32 m = P.m[i].m, mu = P.m[i].mu;
+            const u32 taddr = tmem + ((u32)(32 * warp) << 16) + (u32)buf * 256u;
+            uint8_t* out = W + (((size_t)i * n_mt + mt) * 128 + 32 * warp + lane) * ((size_t)n_nt * kN) + (size_t)nt * kN;
+#pragma unroll 1
+            for (int c0 = 0; c0 < kN; c0 += 32) {
+                u32 r[32];
+                tmem_ld32(taddr + (u32)c0, r);
+                u32 w[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    w[g] = 0;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {  // sums below 2^31: the quotient estimate is at most one short
+                        u32 v = r[4 * g + e] - __umulhi(r[4 * g + e], mu) * m;
+                        v = v >= m ? v - m : v;
+                        w[g] |= v << (8 * e);
+                    }
+                }
+                *(uint4*)(out + c0) = make_uint4(w[0], w[1], w[2], w[3]);
+                *(uint4*)(out + c0 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+            }
+            fence_before();
+            named_sync(kBarEpi, kEpi);  // every lane of the set read
+            if (tid == 0) arrive(smem_u32(&s_tfree[buf]));
+        }
+    }
+    // teardown: every role has left its loop (on abort, after a bounded wait)
+    fence_before();
+    __syncthreads();
+    fence_after();
+    if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+
+// C [rows][cols] from W: a thread combines four columns, stored through shared memory so
+// that a warp writes consecutive words.
+__global__ void __launch_bounds__(256) k_rns_combine(const uint8_t* __restrict__ W, u64* __restrict__ C, int rows,
+                                                     int cols, size_t plane, size_t pitch,
+                                                     const __grid_constant__ Params P) {
+    __shared__ __align__(16) u64 so[1024];
+    const int c0 = blockIdx.x * 1024, c = c0 + 4 * threadIdx.x;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {
+        if (c < cols) {  // pitch is a multiple of 256: the four bytes are inside the row
+            const uint8_t* src = W + (size_t)row * pitch + c;
+            u32 k[4] = {0, 0, 0, 0};
+            u64 lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+            constexpr int kU = 4;  // moduli whose bytes are in flight together
+            for (int i0 = 0; i0 < P.n; i0 += kU, src += kU * plane) {
+                u32 w4[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u) w4[u] = i0 + u < P.n ? __ldcs((const u32*)(src + u * plane)) : 0u;
+#pragma unroll
+                for (int u = 0; u < kU; ++u) {
+                    const Mod& md = P.m[i0 + u];  // zeros past P.n (kMaxMod is a multiple of kU)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const u32 w = (w4[u] >> (8 * e)) & 255u;
+                        k[e] += w * md.recip;
+                        lo[e] += (u64)w * md.mq_lo;
+                        hi[e] += (u64)w * md.mq_hi;
+                    }
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const u32 kk = (k[e] + 8192u) >> 27;
+                lo[e] += (u64)kk * P.nm_lo;  // lo, hi < 21 * 256 * 2^32 < 2^45
+                hi[e] += (u64)kk * P.nm_hi;
+                u64 x = mul_shoup_lazy(hi[e], P.r32, P.r32q, P.q) + lo[e];  // below 2 q + 2^45
+                x -= __umul64hi(x, P.mu) * P.q;
+                x = x >= P.q ? x - P.q : x;
+                so[4 * threadIdx.x + e] = x >= P.q ? x - P.q : x;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int o = threadIdx.x + 256 * e;
+            if (c0 + o < cols) C[(size_t)row * cols + c0 + o] = so[o];
+        }
+        __syncthreads();
+    }
+}
+
+// moduli whose product exceeds 2 inner (q - 1)^2 with a little to spare (0: not enough of them)
+int moduli_for(u32 inner, u64 q) {
+    const double need = 1.05 + std::log2((double)inner) + 2.0 * std::log2((double)(q - 1));
+    double have = 0;
+    for (int n = 0; n < kMaxMod; ++n) {
+        have += std::log2((double)kModuli[n]);
+        if (have > need) return n + 1;
+    }
+    return 0;
+}
+
+// Where the residue system is faster than the byte planes, by moduli of nb bytes (ms, planes
+// against residues, n x n x n): nb <= 3 has at most 9 products against 6 to 9 and an extra
+// combining pass; nb = 4 (32 bits) n = 1024 0.096 / 0.102, n = 2048 0.239 / 0.205, n = 4096
+// 1.052 / 0.834; nb = 5 (35 bits) n = 256 0.084 / 0.078, n = 4096 1.542 / 0.894; nb = 8
+// (60 bits) n = 64 0.096 / 0.082, n = 4096 3.653 / 1.399.
+bool worthwhile(u32 rows, u32 inner, u32 cols, u64 q) {
+    if (q <= (1ull << 24) || q >= (1ull << 62) || inner > (u32)kMaxInner || !moduli_for(inner, q)) return false;
+    if (q <= (1ull << 32) && (double)rows * inner * cols < 2147483648.0) return false;
+    return (u64)((rows + 127) / 128) * ((cols + kN - 1) / kN) < (1ull << 26);
+}
+
+Params make_params(u32 inner, u64 q) {
+    Params P{};
+    P.n = moduli_for(inner, q);
+    u64 mq = 1 % q;  // M mod q
+    for (int i = 0; i < P.n; ++i) mq = (u64)((u128)mq * (u64)kModuli[i] % q);
+    for (int i = 0; i < P.n; ++i) {
+        const u32 m = (u32)kModuli[i];
+        Mod& md = P.m[i];
+        u64 oq = 1 % q;
+        u32 om = 1 % m, inv = 1;
+        for (int j = 0; j < P.n; ++j)
+            if (j != i) {
+                oq = (u64)((u128)oq * (u64)kModuli[j] % q);
+                om = om * (u32)kModuli[j] % m;
+            }
+        while (om * inv % m != 1) ++inv;
+        md.m = m;
+        md.mu_small = (u32)(((1ull << 32) + m - 1) / m);
+        md.mu = (u32)((1ull << 32) / m);
+        u32 ra = 1 % m, rb = inv % m;
+        for (int j = 0; j < 8; ++j) {
+            (j < 4 ? md.a_lo : md.a_hi) |= ra << (8 * (j & 3));
+            (j < 4 ? md.b_lo : md.b_hi) |= rb << (8 * (j & 3));
+            ra = ra * 256 % m;
+            rb = rb * 256 % m;
+        }
+        md.recip = (1u << 27) / m;
+        md.mq_lo = (u32)oq;
+        md.mq_hi = (u32)(oq >> 32);
+    }
+    P.q = q;
+    P.mu = ~0ull / q;
+    P.r32 = (1ull << 32) % q;
+    P.r32q = (u64)(((u128)P.r32 << 64) / q);
+    const u64 nm = mq ? q - mq : 0;
+    P.nm_lo = (u32)nm;
+    P.nm_hi = (u32)(nm >> 32);
+    return P;
+}
+
+int32_t run(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 cols, u64 q, cudaStream_t st) {
+    const Params P = make_params(inner, q);
+    const int n_mt = (int)((rows + 127) / 128), n_nt = (int)((cols + kN - 1) / kN), n_kb = (int)((inner + 31) / 32);
+    int dev = 0, n_sm = 0;
+    CKKS_CUDA_TRY(cudaGetDevice(&dev));
+    CKKS_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+    const size_t plane = (size_t)n_mt * 128 * n_nt * kN;
+    return ptc::timed(dev, st, [&](int* err, auto packed) -> int32_t {
+        Workspace<uint8_t> ap, bp, w;
+        int32_t rc;
+        if ((rc = ap.alloc((size_t)P.n * n_mt * n_kb * kATile, st)) ||
+            (rc = bp.alloc((size_t)P.n * n_nt * n_kb * kBTile, st)) || (rc = w.alloc((size_t)P.n * plane, st)))
+            return rc;
+        const size_t threads = ((size_t)n_mt * 128 + (size_t)n_nt * kN) * 2 * n_kb, blocks = (threads + 255) / 256;
+        const size_t cap = (size_t)n_sm * 16;
+        k_rns_pack<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(lhs, rhs, ap.p, bp.p, (int)rows, (int)inner,
+                                                                            (int)cols, n_mt, n_nt, n_kb,
+                                                                            inner % 2 == 0 && ((uintptr_t)lhs & 15) == 0, P);
+        CKKS_CUDA_TRY(cudaGetLastError());
+        if ((rc = packed())) return rc;
+        CKKS_CUDA_TRY(cudaFuncSetAttribute(k_rns_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        const int n_tiles = n_mt * n_nt * P.n;
+        k_rns_gemm<<<n_tiles < n_sm ? n_tiles : n_sm, kThreads, kSmemBytes, st>>>(ap.p, bp.p, w.p, n_mt, n_nt, n_kb, P,
+                                                                                 err);
+        CKKS_CUDA_TRY(cudaGetLastError());
+        const dim3 g((cols + 1023) / 1024, rows < 65535 ? rows : 65535);
+        k_rns_combine<<<g, 256, 0, st>>>(w.p, out, (int)rows, (int)cols, plane, (size_t)n_nt * kN, P);
+        CKKS_CUDA_TRY(cudaGetLastError());
+        return CKKS_OK;
+    });
+}
+
+}  // namespace rns
 
 int32_t check_dims(uint32_t rows, uint32_t inner, uint32_t cols, uint64_t q, const char* who) {
     // the reference asserts non-empty operands and a modulus above one (ccmm/park.rs:1489-1505)
@@ -514,6 +939,7 @@ int32_t ckks_park_mod_pp_mm_with_backend(const uint64_t* lhs, const uint64_t* rh
     if (backend == CKKS_PARK_TENSOR_CORES) {
         CKKS_CHECK_ARG(tc_ok, "ckks_park_mod_pp_mm: the tensor-core backend needs a compute capability 10.0 device "
                               "and fewer than 2^31 output tiles");
+        if (rns::worthwhile(rows, inner, cols, modulus)) return rns::run(lhs, rhs, out, rows, inner, cols, modulus, st);
         return ptc::run(lhs, rhs, out, rows, inner, cols, modulus, st);
     }
     CKKS_CHECK_ARG(backend == CKKS_PARK_CUDA_CORES, "ckks_park_mod_pp_mm: unknown backend");

@@ -1,0 +1,42 @@
+"""The residue-system form of the tensor-core Park product at the edges of its rule (moduli
+around 2^24, 2^32 and 2^62, inner sums around 33,024 terms), of its tiles (128 rows, 256 columns,
+32-deep steps in stages of four) and of its sums (all zeros, all q - 1), against the 192-bit
+CUDA-core sums and the oracle."""
+import numpy as np
+import pytest
+
+import ckks_b200 as cb
+
+pytestmark = pytest.mark.gpu
+
+
+def check(oracle, a, b, q):
+    da, db = cb.as_u64_tensor(a), cb.as_u64_tensor(b)
+    got = cb.to_numpy_u64(cb.park_mod_pp_mm(da, db, q, backend="tensor_cores"))
+    assert np.array_equal(got, cb.to_numpy_u64(cb.park_mod_pp_mm(da, db, q, backend="cuda_cores")))
+    assert np.array_equal(got[:2], oracle.park_mod_pp_mm(a[:2], b, q))
+
+
+@pytest.mark.parametrize("q", [1 << 24, (1 << 24) + 1, 1 << 32, (1 << 32) + 1, 0x7ffff6001, (1 << 61) - 1, (1 << 62) - 57, 1 << 62])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (128, 32, 256), (129, 33, 257), (3, 129, 1030), (300, 161, 5)])
+def test_shapes_and_moduli(oracle, cuda, q, shape):
+    r, k, c = shape
+    rng = np.random.default_rng(r + k + c)
+    check(oracle, rng.integers(0, 2**64, (r, k), dtype=np.uint64), rng.integers(0, 2**64, (k, c), dtype=np.uint64), q)
+
+
+@pytest.mark.parametrize("inner", [33024, 33025])
+def test_longest_inner_sums(oracle, cuda, inner):
+    q = 0x7ffff6001
+    full = np.full((2, inner), q - 1, np.uint64)
+    check(oracle, full, np.full((inner, 3), q - 1, np.uint64), q)
+    check(oracle, full, np.zeros((inner, 3), np.uint64), q)
+
+
+def test_four_byte_modulus_above_the_size_line(cuda):
+    q, n = (1 << 24) + 43, 1300
+    rng = np.random.default_rng(n)
+    a, b = (cb.as_u64_tensor(rng.integers(0, q, (n, n), dtype=np.uint64)) for _ in range(2))
+    import torch
+    assert torch.equal(cb.park_mod_pp_mm(a, b, q, backend="tensor_cores"),
+                       cb.park_mod_pp_mm(a, b, q, backend="cuda_cores"))

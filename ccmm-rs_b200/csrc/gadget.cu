@@ -8,8 +8,10 @@
 // residue = value mod B; digit = residue - B if residue >= B/2;
 // value = (value - digit) / B, bounded_gadget.rs:75-118).
 #include <map>
+#include <type_traits>
 
 #include "kernels.cuh"
+#include "ntt_core.cuh"
 
 namespace {
 
@@ -21,7 +23,14 @@ struct PrefixConst {
     u64* d_q_words = nullptr;  // [W]
     int W = 0;
     u32 bits = 0;
+    // direct CRT (k_*_cols): columns of 25 bits. NC columns (0: the prefix is too wide);
+    // d_inv [2][q_limbs]: (Q / q_i)^-1 mod q_i and its Shoup companion; d_cols [q_limbs + 2][NC]:
+    // the signed columns of Q / q_i and of Q, the unsigned ones of floor(Q / 2)
+    int NC = 0, pieces = 2;
+    u64* d_inv = nullptr;
+    double* d_cols = nullptr;
 };
+constexpr int kColumnSizes[] = {8, 16, 24, 32, 40, 50};
 
 std::mutex g_prefix_mutex;
 std::map<std::pair<const ckks_ctx*, u32>, PrefixConst> g_prefix;
@@ -39,6 +48,62 @@ void mul_small_add(std::vector<u64>& x, u64 m, u64 a) {
         w = (u64)t;
         carry = t >> 64;
     }
+}
+
+u64 mulmod_host(u64 a, u64 b, u64 q) { return (u64)((u128)a * b % q); }
+
+// Constants of the direct CRT of a prefix (Q, floor(Q/2) as words).
+int32_t column_const(ckks_ctx* ctx, u32 q_limbs, const std::vector<u64>& Q, const std::vector<u64>& half,
+                     PrefixConst* pc) {
+    for (int nc : kColumnSizes)
+        if (!pc->NC && 25 * nc >= (int)pc->bits + 2) pc->NC = nc;
+    if (!pc->NC) return CKKS_OK;
+    const int NC = pc->NC;
+    std::vector<u64> inv(2 * (size_t)q_limbs);
+    std::vector<double> cols((size_t)(q_limbs + 2) * NC);
+    auto columns = [&](const std::vector<u64>& x, double* dst, bool sgn) {
+        int carry = 0;
+        for (int c = 0; c < NC; ++c) {
+            const int bit = 25 * c, w = bit / 64, o = bit % 64;
+            u64 v = w < (int)x.size() ? x[w] >> o : 0;
+            if (o > 39 && w + 1 < (int)x.size()) v |= x[w + 1] << (64 - o);
+            int d = (int)(v & ((1u << 25) - 1)) + carry;
+            carry = sgn && d >= (1 << 24);
+            dst[c] = (double)(d - (carry << 25));
+        }
+    };
+    pc->pieces = 2;
+    for (u32 i = 0; i < q_limbs; ++i) {
+        const u64 qi = ctx->moduli[i];
+        if (qi >= (1ull << 50)) pc->pieces = 3;
+        std::vector<u64> quo = Q;  // Q / q_i (exact)
+        u128 r = 0;
+        for (int w = (int)Q.size() - 1; w >= 0; --w) {
+            const u128 cur = (r << 64) | quo[w];
+            quo[w] = (u64)(cur / qi);
+            r = cur % qi;
+        }
+        columns(quo, cols.data() + (size_t)i * NC, true);
+        u64 m = 1 % qi, e = qi - 2, v = 1;  // (Q / q_i mod q_i)^(q_i - 2)
+        for (u32 j = 0; j < q_limbs; ++j)
+            if (j != i) m = mulmod_host(m, ctx->moduli[j] % qi, qi);
+        for (; e; e >>= 1, m = mulmod_host(m, m, qi))
+            if (e & 1) v = mulmod_host(v, m, qi);
+        inv[i] = v % qi;
+        inv[q_limbs + i] = shoup_quotient_host(inv[i], qi);
+    }
+    columns(Q, cols.data() + (size_t)q_limbs * NC, true);
+    columns(half, cols.data() + (size_t)(q_limbs + 1) * NC, false);
+    if (cudaMalloc(&pc->d_inv, inv.size() * 8) != cudaSuccess || cudaMalloc(&pc->d_cols, cols.size() * 8) != cudaSuccess ||
+        cudaMemcpy(pc->d_inv, inv.data(), inv.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(pc->d_cols, cols.data(), cols.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(pc->d_inv);
+        cudaFree(pc->d_cols);
+        ckks_set_error("out of device memory for gadget constants");
+        return CKKS_ERR_OOM;
+    }
+    return CKKS_OK;
 }
 
 int32_t prefix_const(ckks_ctx* ctx, u32 q_limbs, PrefixConst* out) {
@@ -86,9 +151,273 @@ int32_t prefix_const(ckks_ctx* ctx, u32 q_limbs, PrefixConst* out) {
     }
     cudaMemcpy(pc.d_half_mr, mr.data(), q_limbs * sizeof(u64), cudaMemcpyHostToDevice);
     cudaMemcpy(pc.d_q_words, qpad.data(), kMaxWords * sizeof(u64), cudaMemcpyHostToDevice);
+    if (int32_t rc = column_const(ctx, q_limbs, Q, half, &pc)) {
+        cudaFree(pc.d_half_mr);
+        cudaFree(pc.d_q_words);
+        return rc;
+    }
     g_prefix[key] = pc;
     *out = pc;
     return CKKS_OK;
+}
+
+// Exact centred CRT of one coefficient in columns of 25 bits on the FP64 pipe, without the
+// mixed-radix chain: with u_i = x_i (Q / q_i)^-1 mod q_i, centred,
+//   x = sum_i u_i (Q / q_i) - k Q,   k = rint(sum_i u_i / q_i).
+// Columns are signed 25-bit digits (|.| <= 2^24) and u_i splits into P such pieces, so a
+// product is at most 2^48 and a column of sums an exact double for kRun limbs; a carry pass
+// then brings every column below 2^25. k comes from a double sum that is off by under 2^-41
+// (at most 64 terms of at most 1/2): only when it lies within 2^-40 of a half is the sign
+// open, and then x is compared with floor(Q/2) exactly. Costs P NC fused multiply-adds a
+// limb, at four times the rate of the 32 x 32 + 64-bit integer one, against the L / 2 modular
+// products and W-word steps a limb of the mixed-radix form: 24 limbs of 50 bits, N = 2^16:
+// digits of 16 polynomials 918 -> 517 us, of one 79 -> 42, decode of four 225 -> 93; integer columns
+// in the same form took 708, 62 and 196.
+// Shared memory (stage_columns): the limbs' constants, then the columns of Q / q_i, of Q and of
+// floor(Q/2) (the last unsigned). Returns x < 0 with col its two's complement columns.
+struct LimbConst {
+    double q, qinv, inv, inv_p;  // (Q / q_i)^-1 mod q_i and its quotient by q_i
+    u64 qi, inv_i, inv_q, pad;   // the same as integers, with the Shoup companion
+};
+template <int NC>
+__device__ __forceinline__ void stage_columns(LimbConst* lc, const NttTab* __restrict__ tabs,
+                                              const u64* __restrict__ inv, const double* __restrict__ cols,
+                                              int q_limbs) {
+    double* sh = reinterpret_cast<double*>(lc + q_limbs);
+    for (int i = threadIdx.x; i < q_limbs; i += blockDim.x) {
+        const u64 q = tabs[i].q, v = inv[i];
+        lc[i] = LimbConst{(double)q, 1.0 / (double)q, (double)v, (double)v / (double)q, q, v, inv[q_limbs + i], 0};
+    }
+    for (int i = threadIdx.x; i < (q_limbs + 2) * NC; i += blockDim.x) sh[i] = cols[i];
+    __syncthreads();
+}
+// carries of 25-bit columns: every column to [-2^24, 2^24], the value unchanged (the last
+// column keeps what is left)
+template <int NC>
+__device__ __forceinline__ void carry_columns(double (&acc)[NC]) {
+    constexpr double kM = 6755399441055744.0 * 33554432.0;  // 1.5 * 2^(52 + 25)
+#pragma unroll
+    for (int c = 0; c + 1 < NC; ++c) {
+        const double hi = __dsub_rn(__dadd_rn(acc[c], kM), kM);  // multiple of 2^25
+        acc[c] = __dsub_rn(acc[c], hi);
+        acc[c + 1] = __fma_rn(hi, 1.0 / 33554432.0, acc[c + 1]);
+    }
+}
+template <int NC, int P>
+__device__ __forceinline__ bool crt_columns(const u64* __restrict__ poly, int log_n, int q_limbs, const LimbConst* lc,
+                                            u32 (&col)[NC]) {
+    constexpr int kRun = P == 2 ? 14 : 9;  // 14 * 2 * 2^48 and 9 * 3 * 2^48 plus a carried column: below 2^53
+    constexpr double kM25 = 6755399441055744.0 * 33554432.0, kS25 = 1.0 / 33554432.0;
+    const double* sh = reinterpret_cast<const double*>(lc + q_limbs);
+    double acc[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+    double frac = 0.0;
+    u64 x[3];  // residues of the next limbs, in flight
+#pragma unroll
+    for (int e = 0; e < 3; ++e) x[e] = e < q_limbs ? __ldg(poly + ((size_t)e << log_n)) : 0;
+    for (int i0 = 0; i0 < q_limbs; i0 += kRun) {
+        const int i1 = min(i0 + kRun, q_limbs);
+#pragma unroll 1
+        for (int i = i0; i < i1; ++i) {
+            const LimbConst& T = lc[i];
+            double p[P];
+            if constexpr (P == 2) {  // q below 2^50
+                const double u = nttf::center(nttf::mulmod(nttf::from_u52(x[0]), T.inv, T.inv_p, T.q), T.q, T.qinv);
+                frac = __fma_rn(u, T.qinv, frac);
+                const double hi = __dsub_rn(__dadd_rn(u, kM25), kM25);
+                p[0] = __dsub_rn(u, hi);
+                p[1] = __dmul_rn(hi, kS25);
+            } else {
+                const u64 v = mul_shoup(x[0], T.inv_i, T.inv_q, T.qi);
+                const i64 u = (i64)(v > (T.qi >> 1) ? v - T.qi : v);
+                frac = __fma_rn((double)u, T.qinv, frac);
+                const i64 c1 = (u + (1 << 24)) >> 25, c2 = (c1 + (1 << 24)) >> 25;
+                p[0] = (double)(int)(u - (c1 << 25));
+                p[1] = (double)(int)(c1 - (c2 << 25));
+                p[2] = (double)(int)c2;
+            }
+            x[0] = x[1], x[1] = x[2];
+            if (i + 3 < q_limbs) x[2] = __ldg(poly + ((size_t)(i + 3) << log_n));
+            const double* Qi = sh + i * NC;
+#pragma unroll
+            for (int c0 = 0; c0 < NC; c0 += 2) {
+                const double2 w = *reinterpret_cast<const double2*>(Qi + c0);
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int j = 0; j < P; ++j)
+                        if (c0 + e + j < NC) acc[c0 + e + j] = __fma_rn(p[j], e ? w.y : w.x, acc[c0 + e + j]);
+            }
+        }
+        if (i1 < q_limbs) carry_columns(acc);
+    }
+    const double k = rint(frac);
+    const double *Q = sh + q_limbs * NC, *H = Q + NC;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = __fma_rn(-k, Q[c], acc[c]);
+    carry_columns(acc);
+    i64 carry = 0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const i64 v = (i64)__double2loint(__dadd_rn(acc[c], 6755399441055744.0)) + carry;
+        col[c] = (u32)v & ((1u << 25) - 1);
+        carry = v >> 25;
+    }
+    bool neg = carry < 0;
+    if (fabs(fabs(__dsub_rn(frac, k)) - 0.5) < 0x1p-40) {  // sign open: |x| against floor(Q/2)
+        bool over = false, decided = false;
+        u32 mag[NC], cy = neg ? 1u : 0u;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const u32 t = (neg ? (~col[c] & ((1u << 25) - 1)) : col[c]) + cy;
+            mag[c] = t & ((1u << 25) - 1);
+            cy = t >> 25;
+        }
+#pragma unroll
+        for (int c = NC - 1; c >= 0; --c) {
+            const u32 h = (u32)H[c];
+            if (!decided && mag[c] != h) {
+                over = mag[c] > h;
+                decided = true;
+            }
+        }
+        if (over) {  // one Q back towards zero
+            i64 cr = 0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const i64 qc = (i64)Q[c], v = (i64)col[c] + cr + (neg ? qc : -qc);
+                col[c] = (u32)v & ((1u << 25) - 1);
+                cr = v >> 25;
+            }
+            neg = !neg;
+        }
+    }
+    return neg;
+}
+
+// Resident CTAs asked of the register allocator: left alone it takes 209 to 255 registers by
+// unrolling every column's loads ahead, and one or two CTAs an SM.
+// Capped: 700-bit digits 27.5 -> 23.8 us (3 polynomials of N = 2^15), 1200-bit decode 104 ->
+// 93 us (4 of N = 2^16); the 1200-bit digits are slower capped (41.6 -> 50.7 us).
+constexpr int col_ctas(int nc, bool digits) { return nc <= 32 ? 4 : digits ? 0 : 3; }
+
+// k_bounded_decompose for prefixes of up to 1248 bits and bases up to 2^39.
+template <int NC, int P>
+__global__ void __launch_bounds__(kT, col_ctas(NC, true)) k_bounded_decompose_cols(const u64* __restrict__ poly, i64* __restrict__ digits,
+                                                               u32* __restrict__ flags, const NttTab* __restrict__ tabs,
+                                                               const u64* __restrict__ inv, const double* __restrict__ cols,
+                                                               int q_limbs, int log_n, int base_log, int D,
+                                                               size_t poly_stride) {
+    extern __shared__ __align__(16) LimbConst lc[];
+    stage_columns<NC>(lc, tabs, inv, cols, q_limbs);
+    const u32 n = 1u << log_n;
+    const u32 c0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c0 >= n) return;
+    u32 col[NC];
+    const bool neg = crt_columns<NC, P>(poly + (size_t)blockIdx.y * poly_stride + c0, log_n, q_limbs, lc, col);
+    const i64 B = (i64)1 << base_log, half = B >> 1;
+    i64* out = digits + ((size_t)blockIdx.y * D << log_n) + c0;
+    u64 buf = 0;
+    int have = 0, j = 0;
+    i64 carry = 0;
+    bool flag = false;
+    auto emit = [&]() {
+        i64 d = (i64)(buf & (u64)(B - 1)) + carry;
+        buf >>= base_log;
+        have -= base_log;
+        carry = d >= half;
+        d -= carry ? B : 0;
+        flag |= d == -half;
+        *out = d;
+        out += n;
+        ++j;
+    };
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        buf |= (u64)col[c] << have;
+        have += 25;
+        while (have >= base_log && j < D) emit();
+        if (j >= D) have = 0, buf = 0;
+    }
+    while (j < D) {  // sign extension
+        buf |= (neg ? (u64)((1u << 25) - 1) : 0ull) << have;
+        have += 25;
+        while (have >= base_log && j < D) emit();
+    }
+    if (flags && flag) {  // list of coefficients holding a -B/2 digit: [count][indices]
+        u32* fl = flags + (size_t)blockIdx.y * (n + 1);
+        fl[1 + atomicAdd(fl, 1u)] = c0;
+    }
+}
+
+// k_crt_to_double for prefixes of up to 1248 bits.
+template <int NC, int P>
+__global__ void __launch_bounds__(kT, col_ctas(NC, false)) k_crt_to_double_cols(const u64* __restrict__ poly, double* __restrict__ out,
+                                                           const NttTab* __restrict__ tabs, const u64* __restrict__ inv,
+                                                           const double* __restrict__ cols, int q_limbs, int log_n,
+                                                           double scale) {
+    extern __shared__ __align__(16) LimbConst lc[];
+    stage_columns<NC>(lc, tabs, inv, cols, q_limbs);
+    const u32 n = 1u << log_n;
+    const u32 c0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c0 >= n) return;
+    u32 col[NC];
+    const bool neg = crt_columns<NC, P>(poly + ((size_t)blockIdx.y * q_limbs << log_n) + c0, log_n, q_limbs, lc, col);
+    if (neg) {  // magnitude
+        u32 cy = 1;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const u32 t = (~col[c] & ((1u << 25) - 1)) + cy;
+            col[c] = t & ((1u << 25) - 1);
+            cy = t >> 25;
+        }
+    }
+    // the four leading nonzero columns (at least 76 bits when they are four), the rest as a sticky bit
+    u128 w = 0;
+    int taken = 0, low = 0;
+    bool sticky = false;
+#pragma unroll
+    for (int c = NC - 1; c >= 0; --c) {
+        if (taken == 4) {
+            sticky |= col[c] != 0;
+        } else if (taken || col[c]) {
+            w = (w << 25) | col[c];
+            ++taken;
+            low = c;
+        }
+    }
+    double r = 0.0;
+    const u64 wh = (u64)(w >> 64), wl = (u64)w;
+    if (!wh && !sticky) {
+        r = ldexp(__ull2double_rn(wl), 25 * low);
+    } else {  // 64 leading bits plus a sticky bit round as the whole value
+        const int shift = 64 - __clzll(wh);
+        u64 lead = shift ? (wh << (64 - shift)) | (wl >> shift) : wl;
+        sticky |= shift && (wl << (64 - shift)) != 0;
+        if (sticky) lead |= 1;
+        r = ldexp(__ull2double_rn(lead), 25 * low + shift);
+    }
+    r = neg ? -r : r;
+    out[(size_t)blockIdx.y * n + c0] = __ddiv_rn(r, scale);
+}
+
+// Calls f.template operator()<NC, P>() for the prefix's column count and pieces.
+template <typename F>
+void with_columns(const PrefixConst& pc, F&& f) {
+    auto pick = [&](auto nc) {
+        constexpr int NC = decltype(nc)::value;
+        if (pc.pieces == 2) f(std::integral_constant<int, NC>{}, std::integral_constant<int, 2>{});
+        else f(std::integral_constant<int, NC>{}, std::integral_constant<int, 3>{});
+    };
+    switch (pc.NC) {
+        case 8: pick(std::integral_constant<int, 8>{}); break;
+        case 16: pick(std::integral_constant<int, 16>{}); break;
+        case 24: pick(std::integral_constant<int, 24>{}); break;
+        case 32: pick(std::integral_constant<int, 32>{}); break;
+        case 40: pick(std::integral_constant<int, 40>{}); break;
+        default: pick(std::integral_constant<int, 50>{});
+    }
 }
 
 // bits [start, start + len) of a two's complement value, len <= 63
@@ -298,9 +627,20 @@ int32_t bounded_decompose_launch(ckks_ctx* ctx, const u64* poly, u32 n_polys, u3
     if (int32_t rc = prefix_const(ctx, q_limbs, &pc)) return rc;
     if (!n_polys) return CKKS_OK;
     dim3 grid((ctx->n + kT - 1) / kT, n_polys);
+    if (pc.NC && base_log <= 39) {
+        const size_t smem = q_limbs * sizeof(LimbConst) + (size_t)(q_limbs + 2) * pc.NC * sizeof(double);
+        with_columns(pc, [&](auto nc, auto np) {
+            k_bounded_decompose_cols<decltype(nc)::value, decltype(np)::value><<<grid, kT, smem, st>>>(
+                poly, digits, flags, ctx->d_tabs, pc.d_inv, pc.d_cols, (int)q_limbs, (int)ctx->log_n, (int)base_log,
+                (int)D, poly_stride);
+        });
+        CKKS_CUDA_TRY(cudaGetLastError());
+        return CKKS_OK;
+    }
 #define CKKS_DECOMP(WW)                                                                                          \
     k_bounded_decompose<WW><<<grid, kT, 0, st>>>(poly, digits, flags, ctx->d_tabs, ctx->garner, pc.d_half_mr,     \
                                                  pc.d_q_words, q_limbs, ctx->L, ctx->log_n, base_log, D, poly_stride)
+    // wider bases and prefixes: mixed radix
     if (pc.W <= 4) CKKS_DECOMP(4);
     else if (pc.W <= 8) CKKS_DECOMP(8);
     else if (pc.W <= 16) CKKS_DECOMP(16);
@@ -331,13 +671,19 @@ int32_t crt_to_double_launch(ckks_ctx* ctx, const u64* poly, u32 n_polys, u32 q_
     if (int32_t rc = prefix_const(ctx, q_limbs, &pc)) return rc;
     if (!n_polys) return CKKS_OK;
     dim3 grid((ctx->n + kT - 1) / kT, n_polys);
+    if (pc.NC) {
+        const size_t smem = q_limbs * sizeof(LimbConst) + (size_t)(q_limbs + 2) * pc.NC * sizeof(double);
+        with_columns(pc, [&](auto nc, auto np) {
+            k_crt_to_double_cols<decltype(nc)::value, decltype(np)::value><<<grid, kT, smem, st>>>(
+                poly, out, ctx->d_tabs, pc.d_inv, pc.d_cols, (int)q_limbs, (int)ctx->log_n, scale);
+        });
+        CKKS_CUDA_TRY(cudaGetLastError());
+        return CKKS_OK;
+    }
 #define CKKS_CRT(WW)                                                                                                \
     k_crt_to_double<WW><<<grid, kT, 0, st>>>(poly, out, ctx->d_tabs, ctx->garner, pc.d_half_mr, pc.d_q_words,       \
                                              q_limbs, ctx->L, ctx->log_n, scale)
-    if (pc.W <= 4) CKKS_CRT(4);
-    else if (pc.W <= 8) CKKS_CRT(8);
-    else if (pc.W <= 16) CKKS_CRT(16);
-    else if (pc.W <= 24) CKKS_CRT(24);
+    if (pc.W <= 24) CKKS_CRT(24);  // prefixes beyond the columns' 1248 bits
     else if (pc.W <= 32) CKKS_CRT(32);
     else if (pc.W <= 48) CKKS_CRT(48);
     else CKKS_CRT(66);
@@ -354,6 +700,8 @@ void gadget_release_ctx(const ckks_ctx* ctx) {
         if (it->first.first == ctx) {
             cudaFree(it->second.d_half_mr);
             cudaFree(it->second.d_q_words);
+            cudaFree(it->second.d_inv);
+            cudaFree(it->second.d_cols);
             it = g_prefix.erase(it);
         } else {
             ++it;

@@ -29,10 +29,12 @@ __device__ __forceinline__ int split_bits(u64 q) { return (65 - __clzll(q - 1)) 
 
 // X [n_ent][2][L][N] (NTT domain) -> Xt [L][N][2][ld] at entries e0.., each word
 // pre-split as (x >> sb) << 32 | (x & mask) when `split`, else canonical.
-// Grid (N/32, n_ent/32 rounded up, 2 L).
+// Grid (N/32, n_ent/32 rounded up, 2 L). With img.m the slots hold A images of ld words
+// instead (AImage): the tile's columns are words of the image (grid y over them), of which
+// those of entries e0 .. e0 + n_ent are written.
 __global__ void __launch_bounds__(kTile * 8) k_to_slot_major(const u64* __restrict__ X, u64* __restrict__ Xt,
                                                              const NttTab* __restrict__ tabs, int n_ent, int e0,
-                                                             int ld, int L, int log_n, int split) {
+                                                             int ld, int L, int log_n, int split, AImage img) {
     __shared__ u64 tile[kTile][kTile + 1];
     const u32 n = 1u << log_n;
     const int l = blockIdx.z >> 1, comp = blockIdx.z & 1;
@@ -42,17 +44,34 @@ __global__ void __launch_bounds__(kTile * 8) k_to_slot_major(const u64* __restri
     const int sb = split_bits(q);
     const u64 mask = (1ull << sb) - 1;
     const int tx = threadIdx.x & (kTile - 1), ty = threadIdx.x / kTile;  // 32 x 8
+    __shared__ int s_ent[kTile];  // entry of each column, within this call's entries (-1: none)
+    if (ty == 0) {
+        const int w = c0 + tx;
+        int e = w < n_ent ? w : -1;
+        if (img.m) {
+            int row, t;
+            img.entry(w, &row, &t);
+            e = row + t * img.m - e0;
+            e = w < ld && row < img.m && e >= 0 && e < n_ent ? e : -1;
+        }
+        s_ent[tx] = e;
+        // a tile without entries (an image written in several calls) has nothing to do
+        if (!__any_sync(0xffffffffu, e >= 0) && tx == 0) s_ent[0] = -2;
+    }
+    __syncthreads();
+    if (s_ent[0] == -2) return;
     for (int r = ty; r < kTile; r += 8) {
-        const int e = c0 + r;
-        if (e < n_ent) {
+        const int e = s_ent[r];
+        if (e >= 0) {
             const u64 x = X[((((size_t)e * 2 + comp) * L + l) << log_n) + s0 + tx];
             tile[r][tx] = split ? ((x >> sb) << 32) | (x & mask) : x;
         }
     }
     __syncthreads();
+    const bool mine = s_ent[tx] >= 0;
     for (int r = ty; r < kTile; r += 8) {
-        const int e = c0 + tx;
-        if (e < n_ent) Xt[((((size_t)l << log_n) + s0 + r) * 2 + comp) * ld + e0 + e] = tile[tx][r];
+        const int e = c0 + tx - (img.m ? e0 : 0);
+        if (mine) Xt[((((size_t)l << log_n) + s0 + r) * 2 + comp) * ld + e0 + e] = tile[tx][r];
     }
     (void)n;
 }
@@ -181,16 +200,18 @@ __global__ void __launch_bounds__(kT, 3) k_ccmm_slot(const u64* __restrict__ At,
 }
 
 int32_t to_slot_major(ckks_ctx* ctx, const u64* X, u64* Xt, u32 n_ent, u32 e0, u32 ld, u32 L, bool split,
-                      cudaStream_t st) {
-    dim3 g(ctx->n / kTile, (n_ent + kTile - 1) / kTile, 2 * L);
+                      const AImage& img, cudaStream_t st) {
+    dim3 g(ctx->n / kTile, ((img.m ? ld : n_ent) + kTile - 1) / kTile, 2 * L);
     k_to_slot_major<<<g, kTile * 8, 0, st>>>(X, Xt, ctx->d_tabs, (int)n_ent, (int)e0, (int)ld, (int)L,
-                                             (int)ctx->log_n, split ? 1 : 0);
+                                             (int)ctx->log_n, split ? 1 : 0, img);
     CKKS_CUDA_TRY(cudaGetLastError());
     return CKKS_OK;
 }
 
 // entry-major transforms of n_ent entries (NTT) written slot-major into Xt
-int32_t build_slot_major(ckks_ctx* ctx, const u64* X, u64* Xt, u32 n_ent, u32 L, bool split, cudaStream_t st) {
+// (img.m: A images of img.words words a slot and component)
+int32_t build_slot_major(ckks_ctx* ctx, const u64* X, u64* Xt, u32 n_ent, u32 L, bool split, const AImage& img,
+                         cudaStream_t st) {
     const size_t ct = (size_t)2 * L * ctx->n;
     u32 chunk = (u32)((size_t(1) << 28) / ct);
     if (chunk < 1) chunk = 1;
@@ -202,7 +223,7 @@ int32_t build_slot_major(ckks_ctx* ctx, const u64* X, u64* Xt, u32 n_ent, u32 L,
     for (u32 e0 = 0; e0 < n_ent; e0 += chunk) {
         const u32 m = n_ent - e0 < chunk ? n_ent - e0 : chunk;
         if ((rc = ntt_forward_launch(ctx, X + (size_t)e0 * ct, buf.p, 2 * m, 0, L, st))) return rc;
-        if ((rc = to_slot_major(ctx, buf.p, Xt, m, e0, n_ent, L, split, st))) return rc;
+        if ((rc = to_slot_major(ctx, buf.p, Xt, m, e0, img.m ? (u32)img.words : n_ent, L, split, img, st))) return rc;
     }
     return CKKS_OK;
 }
@@ -221,13 +242,14 @@ int32_t ccmm_structured_launch(ckks_ctx* ctx, const ckks_ksk* key, const u64* A,
     Workspace<u64> At, Bt;
     Workspace<int> terr;
     int32_t rc;
-    if ((rc = At.alloc(slots * 2 * m * kd, st)) || (rc = Bt.alloc(slots * 2 * kd * nd, st))) return rc;
+    const AImage none(0, 0), img = use_tc ? AImage((int)m, (int)kd) : none;
+    if ((rc = At.alloc(slots * 2 * (use_tc ? (size_t)img.words : (size_t)m * kd), st)) || (rc = Bt.alloc(slots * 2 * kd * nd, st))) return rc;
     if (use_tc) {
         if ((rc = terr.alloc(1, st))) return rc;
         CKKS_CUDA_TRY(cudaMemsetAsync(terr.p, 0, sizeof(int), st));
     }
-    if ((rc = build_slot_major(ctx, A, At.p, m * kd, L, !use_tc, st))) return rc;
-    if ((rc = build_slot_major(ctx, B, Bt.p, kd * nd, L, !use_tc, st))) return rc;
+    if ((rc = build_slot_major(ctx, A, At.p, m * kd, L, !use_tc, img, st))) return rc;
+    if ((rc = build_slot_major(ctx, B, Bt.p, kd * nd, L, !use_tc, none, st))) return rc;
     // output columns per chunk: slot-major products plus entry-major quadratic parts within about 2^31 words
     u32 cc = (u32)((size_t(1) << 31) / (slots * 3 * m * 2));
     if (cc > 2) cc &= ~1u;  // whole column pairs per thread

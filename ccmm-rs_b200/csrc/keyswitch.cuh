@@ -108,8 +108,21 @@ int32_t fft_stage_launch(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_rot, 
 // ciphertexts [2][L][N] at the key's level L; C one level down.
 int32_t ccmm_structured_launch(ckks_ctx* ctx, const ckks_ksk* key, const u64* A, const u64* B, u64* C, u32 m, u32 kd,
                                u32 nd, cudaStream_t st);
+// One component of a slot's A in the tensor cores' K-major core-matrix order: row groups of
+// 8 rows (of m rows when m < 8), K chunks of two inner indices, row, inner index.
+struct AImage {
+    int m, rows, chunks, words;
+    CKKS_HD AImage(int m_, int kd) : m(m_), rows(m_ < 8 ? m_ : 8), chunks((kd + 1) / 2),
+                                     words((m_ + 7) / 8 * ((kd + 1) / 2) * rows * 2) {}
+    // row r and inner index t of word w (r may reach past m, t past kd: padding)
+    CKKS_HD void entry(int w, int* r, int* t) const {
+        const int row = (w >> 1) % rows, x = (w >> 1) / rows;
+        *r = x / chunks * 8 + row;
+        *t = 2 * (x % chunks) + (w & 1);
+    }
+};
 // Per-(limb, slot) products of the structured CCMM on the INT8 tensor cores
-// (ccmm_tc.cu): At, Bt slot-major canonical residues, m, kd <= 64.
+// (ccmm_tc.cu): At A images [2][words] a slot, Bt slot-major canonical residues, m, kd <= 64.
 bool ccmm_tc_supported(const ckks_ctx* ctx, u32 m, u32 kd);
 int32_t ccmm_slot_tc_launch(ckks_ctx* ctx, const u64* At, const u64* Bt, u64* Ct, u32 L, u32 m, u32 kd, u32 nd,
                             u32 c_begin, u32 nc, int* err, cudaStream_t st);

@@ -152,17 +152,26 @@ def _u64(a):
 
 
 def _dptr(t):
-    """Device pointer of a contiguous CUDA tensor."""
-    import torch
+    """Device pointer of a contiguous CUDA tensor (an int: the signatures take void pointers)."""
     assert t.is_cuda and t.is_contiguous(), "expected a contiguous CUDA tensor"
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_raw_stream = None
 
 
 def _stream(stream):
-    if stream is None:
+    """The caller's stream, or torch's current one of the current device: asked by its raw
+    handle, since building a Stream object on every call costs more than a launch."""
+    global _raw_stream
+    if stream is not None:
+        return stream
+    if _raw_stream is None:
         import torch
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    return ctypes.c_void_p(stream)
+        torch.cuda.current_stream()  # initialises CUDA
+        get, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        _raw_stream = lambda: get(device())  # noqa: E731
+    return _raw_stream()
 
 
 def as_u64_tensor(a, device="cuda"):

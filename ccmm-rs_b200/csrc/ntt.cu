@@ -798,46 +798,51 @@ k_fwd2_relin(const u64* __restrict__ mid, const u64* __restrict__ key, const u64
     const int limb = blockIdx.z;
     const int log_n = LOG_M + log_a;
     const NttTab& T = tabs[limb];
-    const double2* tab = stage_table_f64(sm + (S::M << log_c), T.fB, S::M);
+    const double2* tab = stage_table_f64(sm + ((S::R1 / S::R2 * S::M) << log_c), T.fB, S::M);
     const double qd = T.qd, qinv = T.qinv;
     double* smd = reinterpret_cast<double*>(sm);
     auto twf = [&](int s, u32 blk) { return tab[(1u << s) + blk]; };
     const int c = tid & (C - 1);
-    const bool act_b = tid < (C << S::LR1);
-    const int g = tid >> log_c;
+    const int g = tid >> log_c;  // the second half's unit: blocks hold C << LR1 threads
     double sb[S::R2], sa[S::R2];
 #pragma unroll
     for (int e = 0; e < S::R2; ++e) sb[e] = sa[e] = 0.0;
-    const bool act_a = tid < (C << S::LR2);
+    // With an odd number of stages the first half has fewer units than threads (R2 < R1): it
+    // then takes kDigits digits at once, each in its own buffer, so every thread has one and
+    // there are two barriers for kDigits digits (N = 2^15: one ciphertext 286 -> 274 us, 1024
+    // of them 74.3 -> 73.1 ms).
+    constexpr int kDigits = S::R1 / S::R2;
+    const int sub = tid / (C << S::LR2), g1 = (tid - sub * (C << S::LR2)) >> log_c;  // first half: digit, row
     const size_t step = (size_t)S::R2 << log_a, digit = (size_t)L << log_n;
-    const u64* in = mid + ((ct * D * L + limb) << log_n) + b0 + c + ((size_t)g << log_a);
+    const u64* in = mid + (((ct * D + sub) * L + limb) << log_n) + b0 + c + ((size_t)g1 << log_a);
     const u64* kb = key + ((size_t)limb << log_n) + b0 + c + ((size_t)brev((u32)g, S::LR1) << log_a);
-    // the next digit's words are loaded before this digit's key words are used, and the key
+    // the next digits' words are loaded before this digit's key words are used, and the key
     // words before the second half's stages, so neither latency stands alone (1024 outputs,
     // 36 digits x 14 limbs of N = 2^15: 102 -> 74 ms)
     u64 raw[S::R1];
-    if (act_a) {
+    if (sub < D) {
 #pragma unroll
         for (int e = 0; e < S::R1; ++e) raw[e] = in[e * step];
     }
     __syncthreads();
-    for (int j = 0; j < D; ++j) {
-        if (act_a) {
+    for (int j0 = 0; j0 < D; j0 += kDigits) {
+        if (j0 + sub < D) {
             double x[S::R1];
 #pragma unroll
             for (int e = 0; e < S::R1; ++e) x[e] = __longlong_as_double((long long)raw[e]);
             nttf::ct_stages<S::LR1>(x, 0, 0, twf, qd);
-            double* o = smd + (g << log_c) + c;
+            double* o = smd + (sub << (LOG_M + log_c)) + (g1 << log_c) + c;
 #pragma unroll
             for (int e = 0; e < S::R1; ++e) o[(S::R2 * e) << log_c] = nttf::center(x[e], qd, qinv);
-            in += digit;
-            if (j + 1 < D) {
+            in += kDigits * digit;
+            if (j0 + kDigits + sub < D) {
 #pragma unroll
                 for (int e = 0; e < S::R1; ++e) raw[e] = in[e * step];
             }
         }
         __syncthreads();
-        if (act_b) {
+#pragma unroll 1
+        for (int j = j0; j < j0 + kDigits && j < D; ++j) {
             constexpr bool kEarly = S::R2 <= 8;  // 16 key pairs beside 16 values would spill
             u64 wb[S::R2], wa[S::R2];
             auto key_words = [&](int e) {
@@ -849,7 +854,7 @@ k_fwd2_relin(const u64* __restrict__ mid, const u64* __restrict__ key, const u64
                 for (int e = 0; e < S::R2; ++e) key_words(e);
             }
             double y[S::R2];
-            const double* o = smd + ((S::R2 * g) << log_c) + c;
+            const double* o = smd + ((j - j0) << (LOG_M + log_c)) + ((S::R2 * g) << log_c) + c;
 #pragma unroll
             for (int e = 0; e < S::R2; ++e) y[e] = o[e << log_c];
             nttf::ct_stages<S::LR2>(y, S::LR1, g, twf, qd);
@@ -870,9 +875,9 @@ k_fwd2_relin(const u64* __restrict__ mid, const u64* __restrict__ key, const u64
                 }
             }
         }
-        __syncthreads();  // smd is rewritten by the next digit
+        __syncthreads();  // the buffers are rewritten by the next digits
     }
-    if (act_b) {
+    {
         const size_t ob0 = ((ct * 2 * L + limb) << log_n) + b0 + c, oa0 = ob0 + ((size_t)L << log_n);
 #pragma unroll
         for (int e = 0; e < S::R2; ++e) {
@@ -1058,7 +1063,7 @@ int32_t ntt_relin_fused_launch(ckks_ctx* ctx, const i64* digits, u64* mid, const
 #define CKKS_RELIN_FUSED(LM)                                                                                  \
     do {                                                                                                      \
         const int lc = pick_log_c<LM>(la, kRelinLogC >= 0 ? kRelinLogC : ctx->ntt_log_c[2]);                  \
-        const size_t smem = (sizeof(u64) << (LM + lc)) + 2 * sizeof(u64) * (1u << LM);                        \
+        const size_t smem = ((LM & 1 ? 2 : 1) * sizeof(u64) << (LM + lc)) + 2 * sizeof(u64) * (1u << LM);     \
         dim3 grid(n_ct, 1u << (la - lc), L);                                                                  \
         constexpr int k4 = LM >= 6 ? 4 : -1, k3 = LM >= 6 ? 3 : -1;                                           \
         auto* f = lc == 4 ? k_fwd2_relin<LM, k4> : lc == 3 ? k_fwd2_relin<LM, k3> : k_fwd2_relin<LM, -1>;     \

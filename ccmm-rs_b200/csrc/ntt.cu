@@ -1285,7 +1285,8 @@ int32_t ntt_autotune(ckks_ctx* ctx, u32 limbs, u32 polys, cudaStream_t st) {
             float ms = 0;
             for (int it = 0; it < 4 && rc == CKKS_OK; ++it) {  // first launch untimed
                 if (it == 1) cudaEventRecord(e0, st);
-                rc = pass(w, log_m[w], a.p, b.p, ctx->d_tabs, lm, limbs, polys, log_o[w], st, InvBase{}, lc);
+                rc = pass(w, log_m[w], a.p, b.p, ctx->d_tabs, lm, limbs, polys, log_o[w], st, InvBase{}, lc, GaloisOut{},
+                          w == 1 ? 32 : 0);  // digits of the usual base 2^32
             }
             if (rc != CKKS_OK) break;
             cudaEventRecord(e1, st);

@@ -1,12 +1,13 @@
 // gadget.cu -- exact gadget decompositions on the GPU.
 //
 // Bounded gadget (grafting/bounded_gadget.rs): per coefficient, exact CRT of
-// the Q residues (mixed-radix Garner with Shoup constants), centring against
-// floor(Q/2) (wide_crt.rs:96-111), conversion to a two's complement integer of
+// the Q residues, centring against floor(Q/2) (wide_crt.rs:96-111), conversion to a two's complement integer of
 // W 64-bit words, then balanced base-2^b digits d_j in [-2^(b-1), 2^(b-1))
 // extracted as chunk_j + carry (identical to the reference loop
 // residue = value mod B; digit = residue - B if residue >= B/2;
-// value = (value - digit) / B, bounded_gadget.rs:75-118).
+// value = (value - digit) / B, bounded_gadget.rs:75-118). The CRT sums columns of
+// 25 bits on the FP64 pipe (k_*_cols); prefixes outside its limits take mixed-radix
+// Garner with Shoup constants.
 #include <map>
 #include <type_traits>
 

@@ -21,7 +21,7 @@ namespace {
 
 constexpr int kT = 256;
 
-// acc[0][l][k] = (l < Lq ? pf_l * base[l][pb(k)] : 0) + sum_j Y[j][l][py(k)] * key[j][l][0][k]
+// acc[0][l][k] = (base ? base[l][pb(k)] : 0) + sum_j Y[j][l][py(k)] * key[j][l][0][k]
 // acc[1][l][k] =                                         sum_j Y[j][l][py(k)] * key[j][l][1][k]
 // py / pb: NTT-domain Galois source maps (k = 0: identity). blockIdx.z batches
 // ciphertexts: Y, base and acc advance by y_stride, b_stride, a_stride words.
@@ -30,9 +30,8 @@ constexpr int kT = 256;
 // words a digit are then read in order and only Y's one word is gathered (N = 2^16,
 // 38 digits, 27 limbs: 341 -> 263 us; 162 us at the copy rate).
 __global__ void __launch_bounds__(kT) k_ks_mac(const u64* __restrict__ Y, const u64* __restrict__ key,
-                                               const u64* __restrict__ base, const u64* __restrict__ pf,
-                                               const u64* __restrict__ pf_q, u64* __restrict__ acc,
-                                               const NttTab* __restrict__ tabs, LimbMap lm, int Lq, int LK, int D,
+                                               const u64* __restrict__ base, u64* __restrict__ acc,
+                                               const NttTab* __restrict__ tabs, LimbMap lm, int LK, int D,
                                                int log_n, u64 perm_y, u64 perm_b, u64 perm_inv, size_t y_stride,
                                                size_t b_stride, size_t a_stride) {
     const u32 n = 1u << log_n;
@@ -77,10 +76,9 @@ __global__ void __launch_bounds__(kT) k_ks_mac(const u64* __restrict__ Y, const 
     ab.fold(q, mu_hi, mu_lo);
     aa.fold(q, mu_hi, mu_lo);
     u64 b = ab.lo;
-    if (base && l < Lq) {  // P b with auxiliary limbs, b without (ordinary RNS key switch)
+    if (base) {  // no auxiliary limbs (ordinary RNS key switch); with them the inverse transform adds P b
         const u32 kb = perm_b ? galois_src(k, perm_b, log_n) : k;
-        const u64 bv = base[((size_t)l << log_n) + kb];
-        b = add_mod(b, pf ? mul_shoup(bv, pf[l], pf_q[l], q) : bv, q);
+        b = add_mod(b, base[((size_t)l << log_n) + kb], q);
     }
     acc[((size_t)l << log_n) + k] = b;
     acc[(((size_t)LK + l) << log_n) + k] = aa.lo;
@@ -372,9 +370,7 @@ int32_t ks_mac_launch(ckks_ctx* ctx, const u64* Y, const u64* key, const u64* ba
         return CKKS_ERR_BAD_ARG;
     }
     dim3 g((ctx->n + kT - 1) / kT, LK, n_ct);
-    k_ks_mac<<<g, kT, 0, st>>>(Y, key, base, with_p ? ctx->d_pmodq : nullptr, with_p ? ctx->d_pmodq + ctx->L : nullptr,
-                               acc, ctx->d_tabs, lm, q_limbs, LK,
-                               D, ctx->log_n, perm_y, perm_b, perm_key ? galois_inverse(perm_key, ctx->n) : 0, ((size_t)D * LK) << ctx->log_n, b_stride,
+    k_ks_mac<<<g, kT, 0, st>>>(Y, key, base, acc, ctx->d_tabs, lm, LK, D, ctx->log_n, perm_y, perm_b, perm_key ? galois_inverse(perm_key, ctx->n) : 0, ((size_t)D * LK) << ctx->log_n, b_stride,
                                ((size_t)2 * LK) << ctx->log_n);
     CKKS_CUDA_TRY(cudaGetLastError());
     return CKKS_OK;
@@ -398,19 +394,27 @@ int32_t rotate_hybrid(ckks_ctx* ctx, const ckks_ksk* key, const u64* ct_in, u64*
     const u32 Lq = key->q_limbs, LK = ksk_limbs(key), D = key->D, n = ctx->n;
     const size_t ct_words = (size_t)2 * Lq * n;
     // ciphertexts are batched through every launch, as many per batch as a few GB allow
-    const size_t per_ct = ct_words * 2 + (size_t)D * LK * n + 4 * (size_t)LK * n + (size_t)D * n;  // words
-    const u32 m_max = (u32)std::max<size_t>(1, std::min<size_t>({(size_t)n_ct, (size_t)65535,
+    const size_t per_ct = ct_words + (size_t)D * LK * n + 4 * (size_t)LK * n + (size_t)D * n;  // words
+    const u32 m_max = (u32)std::max<size_t>(1, std::min<size_t>({(size_t)n_ct, (size_t)(65535 / (D > 2 ? D : 2)),
                                                                    ((size_t)4 << 30) / (per_ct * 8)}));
     Workspace<u64> ws;
     Workspace<i64> dg;
     int32_t rc;
     if ((rc = ws.alloc((size_t)m_max * (per_ct - (size_t)D * n), st)) || (rc = dg.alloc((size_t)m_max * D * n, st)))
         return rc;
-    u64* sct = ws.p;                               // sigma(ct) [m][2][Lq][N]
-    u64* s_hat = sct + (size_t)m_max * ct_words;   // NTT(sigma(ct)) [m][2][Lq][N]; the b parts are the base
-    u64* Y = s_hat + (size_t)m_max * ct_words;     // [m][D][LK][N]
-    u64* acc = Y + (size_t)m_max * D * LK * n;     // [m][2][LK][N]
-    u64* Z = acc + (size_t)m_max * 2 * LK * n;     // [m][2][LK][N]
+    u64* sct = ws.p;                            // sigma(ct) [m][2][Lq][N]
+    u64* Y = sct + (size_t)m_max * ct_words;    // [m][D][LK][N]
+    u64* acc = Y + (size_t)m_max * D * LK * n;  // [m][2][LK][N]
+    u64* Z = acc + (size_t)m_max * 2 * LK * n;  // [m][2][LK][N]
+    // P sigma(b) is added to the b components at the end of the inverse transform: no
+    // transform of sigma(b) (one rotation at N = 2^16, 24 + 3 limbs: 3.5 % less; 64 chains of
+    // product and rotation at N = 2^12, three limbs: 386 -> 368 us)
+    InvBase ib;
+    ib.b = sct;
+    ib.b_stride = ct_words;
+    ib.q_limbs = Lq;
+    ib.pf = ctx->d_pmodq;
+    ib.pf_q = ctx->d_pmodq + ctx->L;
     const LimbMap lq = LimbMap::range(0, Lq), lqp = LimbMap::qp(ctx, Lq);
     for (u32 c0 = 0; c0 < n_ct; c0 += m_max) {
         const u32 m = n_ct - c0 < m_max ? n_ct - c0 : m_max;
@@ -421,11 +425,9 @@ int32_t rotate_hybrid(ckks_ctx* ctx, const ckks_ksk* key, const u64* ct_in, u64*
                                            ct_words)))
             return rc;
         if ((rc = ntt_forward_digits_launch(ctx, dg.p, Y, D * m, lqp, LK, st, key->base_log))) return rc;
-        if ((rc = ntt_forward_launch_map(ctx, sct, s_hat, 2 * m, lq, Lq, st))) return rc;
-        if ((rc = ks_mac_launch(ctx, Y, key->d_entries, s_hat, acc, Lq, D, true, 0, 0, st, key->exponent, m,
-                                ct_words)))
+        if ((rc = ks_mac_launch(ctx, Y, key->d_entries, nullptr, acc, Lq, D, true, 0, 0, st, key->exponent, m)))
             return rc;
-        if ((rc = ntt_inverse_launch_map(ctx, acc, Z, 2 * m, lqp, LK, st))) return rc;
+        if ((rc = ntt_inverse_base_launch(ctx, acc, Z, 2 * m, lqp, LK, ib, st))) return rc;
         if ((rc = mod_down_launch(ctx, Z, out, 2 * m, Lq, st))) return rc;
     }
     return CKKS_OK;

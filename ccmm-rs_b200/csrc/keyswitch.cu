@@ -5,7 +5,7 @@
 //   sigma_k on (b, a)                         coefficient-domain automorphism
 //   digits of sigma(a)                        bounded gadget (exact CRT) or RNS blocks
 //   Y[j][l] = NTT_l(lift(d_j))                one fused lift + forward NTT launch
-//   acc_b[l] = (P mod q_l) NTT(sigma b)[l] + sum_j Y[j][l] key_b[j][l]
+//   acc_b[l] = sum_j Y[j][l] key_b[j][l]  (P sigma(b) is added by the inverse transform)
 //   acc_a[l] =                               sum_j Y[j][l] key_a[j][l]
 //   INTT, exact ModDown by P                  (ring/auxiliary_modulus.rs:89-171)
 // The MAC accumulates exact 128-bit sums of products and reduces once per

@@ -11,7 +11,8 @@
 //     s00 (unit 1), s01 (unit 2^25) and s11 (unit 2^50): a term adds at most
 //     2^48, 2 * 2^48 and 2^48 units, so s01 is exact for 16 terms and s00, s11
 //     for 32. center() of each (one FMA, exact: the result is an integer below
-//     2^53) folds them into s00 every kFold terms.
+//     2^53) folds s01 into s00 every kFold terms and s11 every 2 kFold, which
+//     leaves s00 room for the centred values it holds (bound at the fold).
 //   P = 3 (q < 2^62): 21-bit pieces in [0, 2^21), nine FMAs into five sums of at
 //     most 3 * 2^42 a term: exact without folding for up to 680 digits.
 // Every residue is the canonical one of the same integer sum, so the words equal
@@ -40,7 +41,7 @@ namespace macf {
 
 constexpr int kJs = 2;        // digits per stage
 constexpr int kStages = 4;    // raw stages (kStages - 1 in flight)
-constexpr int kFold = 14;     // terms between folds of s01 (every second fold takes s00 and s11)
+constexpr int kFold = 12;     // terms between folds of s01 (every second fold takes s00 and s11)
 // Threads and resident CTAs: two CTAs of 256 hide each other's stage barriers (5 keys, 6
 // ciphertexts: 271 -> 196 us against one CTA of 512; equal at 16 ciphertexts); the
 // three-piece form keeps one CTA of 512, which splits its words once for twice the keys
@@ -270,9 +271,10 @@ __global__ void __launch_bounds__(kMaxThreads<P>, 512 / kMaxThreads<P>) k_mac_f6
         for (; t < t_end; ++t) step(t);
         if (t >= steps) break;
         if constexpr (P == 2) {
-            // s01 after kFold terms (14 * 2^49 < 2^53 units), s00 and s11 after 2 kFold: until then s00
-            // holds a centred value (q/2 < 2 * 2^48), 28 * 2^48 and one centred s01: at most 32 * 2^48 = 2^53.
-            // center(s11): |s11| / q < 7 q < 2^52.9, so the quotient is off by under 1.8 and |r| < 2.3 q.
+            // s01 after kFold terms (12 * 2^49 < 2^53 units), s00 and s11 after 2 kFold: until s00 is centred
+            // it holds a centred start, 24 products and the centred s01 of both folds. A centred value is at
+            // most q/2 < 2 * 2^48 and the quotient's rounding (2^26 for s01): below 31 * 2^48 < 2^53.
+            // center(s11): |s11| / q < 6 q < 2^52.6, so the quotient is off by under 1.8 and |r| < 2.3 q.
 #pragma unroll
             for (int i = 0; i < C; ++i)
 #pragma unroll

@@ -59,3 +59,28 @@ def test_tensor_core_mac_corrections_in_a_full_group(cuda):
     ctx.tensor_cores = False
     assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d)))
 
+
+def test_two_piece_sums_at_their_bound(oracle, cuda):
+    """A ciphertext of one constant whose base-2^25 digits all lie just above -2^24 and an uploaded
+    key whose words' low pieces do: over 57 digits the unit sums grow with one sign through two
+    full folds, and the centred high-piece sums of some slots with them."""
+    q, p = chain(1 << 8, (50,) * 29, (60,))
+    ctx = cb.Context(8, q, p)
+    n, base_log = ctx.n, 25
+    rng = np.random.default_rng(25)
+    k = ctx.rotation_exponent_left(1)
+    shape = (cb.KeySwitchKey.hybrid_generate(ctx, len(q), base_log, k, np.ones(n, np.int8), seed=1).info()[0],
+             len(q) + 1, 2, n)
+    entries = np.empty(shape, np.uint64)
+    for i, m in enumerate(q + p):
+        high = rng.integers(0, int(m) >> 26, (shape[0], 2, n), dtype=np.int64)
+        entries[:, i] = ((high << 25) - (1 << 24) + rng.integers(0, 1 << 8, high.shape)) % int(m)
+    key = cb.KeySwitchKey.hybrid_upload(ctx, len(q), base_log, k, entries)
+    value = sum((-(1 << 24) + 1 + 2 * int(r)) << (base_log * j) for j, r in enumerate(rng.integers(0, 1 << 7, 57)))
+    ct = np.zeros((1, 2, len(q), n), np.uint64)
+    ct[0, 1, :, 0] = [value % int(m) for m in q]
+    d = cb.as_u64_tensor(ct)
+    got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, [key], d))
+    ctx.tensor_cores = False
+    assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, [key], d)))
+    assert np.array_equal(got[0, 0], oracle.hybrid_rotate(q, p, entries, k, base_log, ct[0]))

@@ -224,8 +224,9 @@ class Context:
     @property
     def last_mac_path(self):
         """Path of the most recent hoisted rotation MAC or CCMM slot product on
-        this context: "tensor_cores", "cuda_cores" or None (neither ran yet)."""
-        return {1: "tensor_cores", 0: "cuda_cores"}.get(int(lib().ckks_ctx_last_mac_path(self.handle)))
+        this context: "tensor_cores", "fp64" (hoisted rotations of few pairs on the
+        FP64 pipe), "cuda_cores" or None (none ran yet)."""
+        return {1: "tensor_cores", 2: "fp64", 0: "cuda_cores"}.get(int(lib().ckks_ctx_last_mac_path(self.handle)))
 
     def autotune(self, limbs, polys, stream=None):
         """Times the NTT passes' tile choices on a limbs x polys batch, keeps the

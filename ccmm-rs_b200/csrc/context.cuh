@@ -80,8 +80,8 @@ struct ckks_ctx {
     // key-switch MAC of bounded hoisted rotations: tcgen05 INT8 tensor cores
     // (when the device has them) or the CUDA-core split-accumulator form
     bool tensor_cores = true;
-    // MAC of the most recent hoisted rotation on this context: 1 tensor cores,
-    // 0 CUDA cores, -1 none yet (diagnostic; read by ckks_ctx_last_mac_path)
+    // MAC of the most recent hoisted rotation on this context: 1 tensor cores, 2 the
+    // FP64 pipe, 0 CUDA cores, -1 none yet (diagnostic; read by ckks_ctx_last_mac_path)
     int last_mac_path = -1;
     // NTT columns per CTA (log2) per pass: forward 1, forward 1 of digits,
     // forward 2, inverse 1, inverse 2; -1 = built-in choice; set by the autotuner

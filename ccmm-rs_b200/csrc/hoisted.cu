@@ -1215,7 +1215,7 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
     // the tensor-core MAC reads the keys' packed set (made on first use)
     const PackedSet* pset = use_tc && !use_f64 ? packed_set_get(ctx, keys, n_keys, st) : nullptr;
     use_tc = pset != nullptr;
-    ctx->last_mac_path = use_tc ? 1 : 0;
+    ctx->last_mac_path = use_tc ? 1 : use_f64 ? 2 : 0;
     const bool with_base = use_tc || use_f64;  // the MAC adds P NTT(b) itself
     u32 G = n_ct >= 4 ? 4 : n_ct;
     if (use_tc) G = n_ct < pset->g_max ? n_ct : pset->g_max;

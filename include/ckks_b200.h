@@ -90,11 +90,12 @@ int32_t ckks_ctx_set_tensor_cores(ckks_ctx* ctx, int32_t enable);
 int32_t ckks_ctx_tensor_cores(const ckks_ctx* ctx);
 /* Which path the most recent hoisted rotation MAC (ckks_rotate_hoisted and the
  * calls built on it) or structured CCMM slot product on this context ran: 1 the
- * tcgen05 INT8 tensor cores, 0 the CUDA cores (tensor cores switched off, at
- * most 160 (ciphertext, key) pairs in a group of up to 16 ciphertexts,
- * RNS-block keys, rings below the tensor-core tile, too little free device
- * memory for the packed key set, or CCMM blocks beyond 64 rows or inner
- * entries), -1 neither yet. Diagnostic only; no counterpart in the reference. */
+ * tcgen05 INT8 tensor cores, 2 the FP64 pipe (hoisted rotations of at most 160
+ * (ciphertext, key) pairs in a group of up to 16 ciphertexts), 0 the CUDA cores
+ * (tensor cores switched off, RNS-block keys, rings below the tensor-core tile,
+ * too little free device memory for the packed key set, or CCMM blocks beyond 64
+ * rows or inner entries), -1 none yet. Diagnostic only; no counterpart in the
+ * reference. */
 int32_t ckks_ctx_last_mac_path(const ckks_ctx* ctx);
 /* Autotuner (no counterpart in the reference, whose NTT has no launch shape):
  * times every admissible columns-per-CTA choice of the five NTT passes

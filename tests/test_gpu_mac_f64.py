@@ -42,9 +42,10 @@ def test_f64_mac_equals_cuda_core_mac(oracle, cuda, log_n, q_bits, p_bits, n_ct,
     q, p, ctx, ks, keys, cts = setup(log_n, q_bits, p_bits, n_ct, range(1, n_keys + 1), base_log, 31 + n_ct, plant)
     d = cb.as_u64_tensor(cts)
     got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d))
-    assert ctx.last_mac_path == "cuda_cores"
+    assert ctx.last_mac_path == "fp64"
     ctx.tensor_cores = False
     assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d)))
+    assert ctx.last_mac_path == "cuda_cores"
     for c, g in {(0, 0), (n_ct - 1, n_keys - 1)}:
         want = oracle.hybrid_rotate(q, p, keys[g].download(), ks[g], base_log, cts[c])
         assert np.array_equal(got[c, g], want), (c, g)
@@ -81,6 +82,8 @@ def test_two_piece_sums_at_their_bound(oracle, cuda):
     ct[0, 1, :, 0] = [value % int(m) for m in q]
     d = cb.as_u64_tensor(ct)
     got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, [key], d))
+    assert ctx.last_mac_path == "fp64"
     ctx.tensor_cores = False
     assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, [key], d)))
+    assert ctx.last_mac_path == "cuda_cores"
     assert np.array_equal(got[0, 0], oracle.hybrid_rotate(q, p, entries, k, base_log, ct[0]))

@@ -265,6 +265,7 @@ def test_tensor_core_mac_equals_cuda_core_mac(oracle, cuda, base_log, q_bits):
                     for _ in range(16)])
     assert ctx.tensor_cores
     tc = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
+    assert ctx.last_mac_path == "tensor_cores"
     ctx.tensor_cores = False
     assert not ctx.tensor_cores
     cc = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
@@ -276,7 +277,7 @@ def test_tensor_core_mac_equals_cuda_core_mac(oracle, cuda, base_log, q_bits):
 
 
 def test_tensor_core_mac_corrections_bit_exact(oracle, cuda):
-    """Tensor-core path (17 keys or more) with planted -B/2 digits: the carry
+    """Tensor-core path (10 ciphertexts, a partial group, by 18 keys) with planted -B/2 digits: the carry
     corrections of the NTT-domain hoisting are applied in the tensor-core
     epilogue and the words equal the oracle's and the CUDA-core MAC's."""
     log_n, n, base_log = 12, 1 << 12, 32
@@ -286,7 +287,7 @@ def test_tensor_core_mac_corrections_bit_exact(oracle, cuda):
     rng = np.random.default_rng(91)
     s = rng.integers(-1, 2, n).astype(np.int8)
     cts = np.stack([np.stack([np.stack([rng.integers(0, m, n, dtype=np.uint64) for m in q]) for _ in range(2)])
-                    for _ in range(3)])
+                    for _ in range(10)])
     Q = 1
     for m in q:
         Q *= m
@@ -297,11 +298,12 @@ def test_tensor_core_mac_corrections_bit_exact(oracle, cuda):
     keys = [cb.KeySwitchKey.hybrid_generate(ctx, len(q), base_log, k, s, seed=700 + i) for i, k in enumerate(ks)]
     assert ctx.tensor_cores
     tc = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
+    assert ctx.last_mac_path == "tensor_cores"
     ctx.tensor_cores = False
     cc = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
     ctx.tensor_cores = True
     assert np.array_equal(tc, cc)
-    for c, g in ((0, 0), (0, 17), (0, 9), (2, 3)):
+    for c, g in ((0, 0), (0, 17), (0, 9), (9, 3)):
         want = oracle.hybrid_rotate(q, p, keys[g].download(), ks[g], base_log, cts[c])
         assert np.array_equal(tc[c, g], want), (c, g)
 
@@ -316,14 +318,16 @@ def test_packed_key_sets_follow_key_lifetimes(oracle, cuda):
     rng = np.random.default_rng(123)
     s = rng.integers(-1, 2, n).astype(np.int8)
     cts = np.stack([np.stack([np.stack([rng.integers(0, m, n, dtype=np.uint64) for m in q]) for _ in range(2)])
-                    for _ in range(2)])
+                    for _ in range(10)])
     ks = [ctx.rotation_exponent_left(r) for r in range(1, 19)]
     keys = [cb.KeySwitchKey.hybrid_generate(ctx, len(q), base_log, k, s, seed=40 + i) for i, k in enumerate(ks)]
     first = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
+    assert ctx.last_mac_path == "tensor_cores"
     for trial in range(2):
         keys[5].close()  # frees the key and every packed set that holds it
         keys[5] = cb.KeySwitchKey.hybrid_generate(ctx, len(q), base_log, ks[5], s, seed=1000 + trial)
         got = host(cb.rotate_hoisted(ctx, keys, dev(cts)))
+        assert ctx.last_mac_path == "tensor_cores"
         want5 = oracle.hybrid_rotate(q, p, keys[5].download(), ks[5], base_log, cts[1])
         assert np.array_equal(got[1, 5], want5)
         assert np.array_equal(got[:, :5], first[:, :5]) and np.array_equal(got[:, 6:], first[:, 6:])

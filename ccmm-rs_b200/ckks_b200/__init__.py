@@ -211,9 +211,9 @@ class Context:
 
     @property
     def tensor_cores(self):
-        """True when bounded hoisted rotations of more than 160 (ciphertext, key)
-        pairs a group run their key-switch MAC, and the structured CCMM its
-        per-slot products (m, k <= 64), on the INT8 tensor cores (enabled by
+        """True when bounded hoisted rotations run their key-switch MAC (groups of
+        few (ciphertext, key) pairs: on the FP64 pipe), and the structured CCMM
+        its per-slot products (m, k <= 64), on the INT8 tensor cores (enabled by
         default where the device has them)."""
         return bool(lib().ckks_ctx_tensor_cores(self.handle))
 

@@ -22,6 +22,7 @@
 #include "ntt_core.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -1186,11 +1187,11 @@ constexpr bool kFoldSigma = CKKS_FOLD_SIGMA != 0;
 #endif
 constexpr bool kFuseModDown = CKKS_FUSE_MODDOWN != 0;
 
-// (ciphertext, key) pairs of a group up to which the MAC runs on the FP64 pipe
-// (mac_f64.cuh). Measured at N=2^16, 24 + 3 limbs, D = 38: the tensor-core MAC takes
-// 21.3-21.5 ms for any number of pairs up to 16 x 32 (its items pad to 32 keys and 16
-// ciphertexts), the FP64 MAC 12.8 ms for 16 x 6 and 30.0 ms for 16 x 16 pairs, so the
-// lines cross near 180. It also needs no packed copy of the keys.
+// (ciphertext, key) pairs of a group up to which the MAC may run on the FP64 pipe
+// (mac_f64.cuh): where it is the faster one, macf::cheaper_than_tc, and where the keys' packed
+// set does not fit and more than 4 ciphertexts share a key slice (16 x 11 pairs at N = 2^16,
+// 24 + 3 limbs: 28.8 ms against 36.7 with 16 x 12 on the CUDA cores; 4 x 24: 20.4 against 16.8).
+// The measurements of both end at 160 pairs.
 constexpr size_t kF64MacPairs = 160;
 
 // Hoisted hybrid rotations of n_ct ciphertexts by n_keys Galois keys (bounded
@@ -1210,16 +1211,19 @@ int32_t rotate_hoisted_ntt(ckks_ctx* ctx, const ckks_ksk* const* keys, u32 n_key
     // otherwise groups of 4 on the CUDA-core tiled MAC.
     bool use_tc = bounded && n >= (u32)tc::kTS && D < 4096 && ctx->tensor_cores && tc_enabled();
     // few (ciphertext, key) pairs a group: the FP64 MAC (rule at kF64MacPairs)
-    const bool use_f64 = use_tc && D <= (u32)macf::kMaxDigits && n >= 16 &&
-                         (n_ct < kGroupMax ? n_ct : kGroupMax) * (size_t)n_keys <= kF64MacPairs;
+    const u32 g_full = n_ct < kGroupMax ? n_ct : kGroupMax;
+    const bool f64_ok = use_tc && D <= (u32)macf::kMaxDigits && n >= 16 && g_full * (size_t)n_keys <= kF64MacPairs;
+    bool use_f64 = f64_ok && macf::cheaper_than_tc(ctx, LimbMap::qp(ctx, Lq), (int)LK, (int)D, (int)k0->base_log,
+                                                   (int)g_full, (int)n_keys);
     // the tensor-core MAC reads the keys' packed set (made on first use)
     const PackedSet* pset = use_tc && !use_f64 ? packed_set_get(ctx, keys, n_keys, st) : nullptr;
     use_tc = pset != nullptr;
+    use_f64 |= f64_ok && !use_tc && g_full > 4;
     ctx->last_mac_path = use_tc ? 1 : use_f64 ? 2 : 0;
     const bool with_base = use_tc || use_f64;  // the MAC adds P NTT(b) itself
     u32 G = n_ct >= 4 ? 4 : n_ct;
     if (use_tc) G = n_ct < pset->g_max ? n_ct : pset->g_max;
-    if (use_f64) G = n_ct < kGroupMax ? n_ct : kGroupMax;
+    if (use_f64) G = g_full;
     const int cap = 1024;
     const LimbMap lqp = LimbMap::qp(ctx, Lq);
     const size_t y_stride = (size_t)D * LK * n, d_stride = (size_t)D * n, f_stride = (size_t)n + 1,

@@ -27,7 +27,7 @@
 // time), the fetches (5 %) or the final reductions (5 %) in timing-only copies shows
 // the FMA loop itself holds the rest. Two-digit unrolling (+4 %), 255 registers at
 // half the warps (+35 %) and row-wise bulk copies (85 cycles a copy: 2.4x the time)
-// were slower. Times by pairs: kF64MacPairs in hoisted.cu.
+// were slower. Times by pairs: cheaper_than_tc.
 //
 // A CTA owns 16 T slots of one limb, every ciphertext of the group and up to 8
 // keys. Rows (ciphertexts, then key components) come in by cp.async, kJs digits
@@ -369,11 +369,43 @@ int32_t launch_c(const ckks_ctx* ctx, Args a, cudaStream_t st) {
     return launch_class<3, C, 2>(a, n3, st);
 }
 
+// ciphertexts a thread sums
+inline int tile_cts(int n_ct) { return n_ct == 1 ? 1 : n_ct > 8 || n_ct % 4 == 0 ? 4 : 2; }
+
 // up to 16 ciphertexts, any number of keys, N >= 16, D <= kMaxDigits, every prime above 2^21
 inline int32_t launch(const ckks_ctx* ctx, const Args& a, cudaStream_t st) {
-    if (a.n_ct == 1) return launch_c<1>(ctx, a, st);
-    if (a.n_ct > 8 || a.n_ct % 4 == 0) return launch_c<4>(ctx, a, st);
-    return launch_c<2>(ctx, a, st);
+    switch (tile_cts(a.n_ct)) {
+        case 1: return launch_c<1>(ctx, a, st);
+        case 2: return launch_c<2>(ctx, a, st);
+        default: return launch_c<4>(ctx, a, st);
+    }
+}
+
+// Whether this MAC takes less time than the tensor-core one for a group of n_ct ciphertexts, by
+// estimates (us) fitted to both on a B200 (ten rings, chains and bases, 140 groups of 40 to 160 pairs).
+// Tensor cores: 5.4 ns a slot and 0.67 ns more for each 4 digits (the base digit with them), for
+// every 32 keys begun, whatever the ciphertexts (within 5 %; up to 20 % more for wide limbs at
+// N = 2^16). This MAC: a cost a slot and digit for every 8 keys begun (fewer than 8 cost
+// (keys + 2) / 10 of that), which grows with the padded ciphertexts and the pieces a prime needs.
+// ms, tensor cores / FP64: N = 2^16, 24 50-bit and three 60-bit limbs, D = 38: 16 x 8 21.3 / 14.6,
+// 16 x 9 21.3 / 28.7; N = 2^15, 14 60-bit limbs, D = 23: 16 x 7 4.61 / 4.57, 16 x 8 4.45 / 4.72,
+// 8 x 20 4.32 / 6.46; N = 2^12, six 50-bit and a 60-bit limb, D = 10: 16 x 9 0.252 / 0.214.
+// Carry corrections (-B/2 digits, D N / B of them expected a ciphertext) cost every slot 3.7 ns here
+// for a ciphertext and 8 keys, 22 ns there for a ciphertext and 32 keys, whose rows share a warp:
+// N = 2^15, 12 50-bit and two 60-bit limbs, base 2^20: 16 x 10 150 / 53 ms, base 2^24 18.7 / 15.2.
+inline bool cheaper_than_tc(const ckks_ctx* ctx, const LimbMap& lm, int LK, int D, int base_log, int n_ct,
+                            int n_keys) {
+    const int tile = tile_cts(n_ct), cts = (n_ct + tile - 1) / tile * tile;
+    const double two = 0.25 + 0.035 * cts;  // pieces of a prime below 2^50
+    const double three = cts > 8 ? 0.1 * cts : cts == 6 ? 0.92 : 0.22 + 0.063 * cts;
+    double limbs = 0;
+    for (int l = 0; l < LK; ++l) limbs += ctx->moduli[lm(l)] < (1ull << 50) ? two : three;
+    const int eights = (n_keys + kKeysMax - 1) / kKeysMax, chunks = (n_keys + 31) / 32;
+    const double keys = n_keys < kKeysMax ? (n_keys + 2) / 10.0 : eights;
+    const double slots = (double)LK * ctx->n, corrections = std::ldexp((double)D * ctx->n, -base_log) * n_ct;
+    const double f64 = 10.0 + limbs * ctx->n * keys * 0.174e-3 * (D + 14) + slots * eights * 3.7e-3 * corrections;
+    const double tc = 40.0 + 1e-3 * slots * chunks * (5.4 + 0.67 * (D / 4 + 1) + 22.0 * corrections);
+    return f64 < tc;
 }
 
 }  // namespace macf

@@ -78,8 +78,8 @@ int32_t ckks_ctx_destroy(ckks_ctx* ctx);
 /* Selects the key-switch MAC of bounded hoisted rotations and the per-slot
  * products of ckks_ccmm_structured (rows and inner dimension <= 64): enable != 0
  * (the default) runs them on the tcgen05 INT8 tensor cores when the device has
- * them (rotation groups of at most 160 (ciphertext, key) pairs, where that MAC's
- * tiles would be mostly padding, on the FP64 pipe), 0 on CUDA cores
+ * them (rotation groups of few (ciphertext, key) pairs, where that MAC's tiles
+ * would be mostly padding, on the FP64 pipe), 0 on CUDA cores
  * (split-operand 64-bit accumulators). All are
  * bit-exact; the switch exists to compare them. No counterpart in the reference
  * (its MAC is the serial loop of ring/ntt_polynomial.rs:211-236, its CCMM the
@@ -90,8 +90,9 @@ int32_t ckks_ctx_set_tensor_cores(ckks_ctx* ctx, int32_t enable);
 int32_t ckks_ctx_tensor_cores(const ckks_ctx* ctx);
 /* Which path the most recent hoisted rotation MAC (ckks_rotate_hoisted and the
  * calls built on it) or structured CCMM slot product on this context ran: 1 the
- * tcgen05 INT8 tensor cores, 2 the FP64 pipe (hoisted rotations of at most 160
- * (ciphertext, key) pairs in a group of up to 16 ciphertexts), 0 the CUDA cores
+ * tcgen05 INT8 tensor cores, 2 the FP64 pipe (at most 160 (ciphertext, key)
+ * pairs in a group of up to 16 ciphertexts, where the sizes and prime widths make
+ * it the faster one or the packed key set does not fit), 0 the CUDA cores
  * (tensor cores switched off, RNS-block keys, rings below the tensor-core tile,
  * too little free device memory for the packed key set, or CCMM blocks beyond 64
  * rows or inner entries), -1 none yet. Diagnostic only; no counterpart in the

@@ -51,6 +51,22 @@ def test_f64_mac_equals_cuda_core_mac(oracle, cuda, log_n, q_bits, p_bits, n_ct,
         assert np.array_equal(got[c, g], want), (c, g)
 
 
+# groups on both sides of the line: it follows the primes' width, the digits, the keys begun and
+# the carry corrections to expect
+@pytest.mark.parametrize("q_bits,n_ct,n_keys,base_log,path", [
+    ((60,) * 6, 16, 8, 32, "fp64"), ((60,) * 6, 16, 9, 32, "tensor_cores"), ((60,) * 6, 5, 24, 32, "tensor_cores"),
+    ((60,) * 6, 16, 9, 20, "fp64"), ((50,) * 6, 16, 9, 32, "fp64"), ((50,) * 20, 16, 9, 36, "tensor_cores"),
+    ((50,) * 6, 1, 33, 32, "fp64"),
+])
+def test_faster_mac_by_width_digits_and_keys(cuda, q_bits, n_ct, n_keys, base_log, path):
+    q, p, ctx, ks, keys, cts = setup(12, q_bits, (60,), n_ct, range(1, n_keys + 1), base_log, 17)
+    d = cb.as_u64_tensor(cts)
+    got = cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d))
+    assert ctx.last_mac_path == path
+    ctx.tensor_cores = False
+    assert np.array_equal(got, cb.to_numpy_u64(cb.rotate_hoisted(ctx, keys, d)))
+
+
 def test_tensor_core_mac_corrections_in_a_full_group(cuda):
     """16 x 18 pairs stay on the tensor-core MAC: its carry corrections against the CUDA-core MAC's."""
     q, p, ctx, ks, keys, cts = setup(12, (50,) * 4, (60,), 16, range(1, 19), 32, 91, plant=True)

@@ -33,7 +33,8 @@
 // reciprocals (each below the true one by under 2^-27: the sum is off by under 2^-14).
 // Packing takes two byte dot products an element and modulus; the GEMM is the persistent
 // kernel below with N = 256 and one accumulator, storing w_i as bytes; one kernel combines
-// the n_mod bytes of an output. n = 4096, 35-bit q: packing 0.17 ms, GEMM 0.54 ms (2.80 POP/s,
+// the n_mod bytes of an output, in slabs of the product whose workspace is bounded. n = 4096,
+// 35-bit q: packing 0.17 ms, GEMM 0.54 ms (2.80 POP/s,
 // 88 % of twice the bf16 rate: the tensor pipe bounds it), combining 0.12 ms; the byte planes
 // took 0.26 and 1.24 ms.
 //
@@ -42,6 +43,7 @@
 // consecutive), staging 16-deep slices of both operands in shared memory; each
 // dot product is summed exactly in 192 bits (any u64 inputs, up to 2^64 terms)
 // and reduced once.
+#include <algorithm>
 #include <cmath>
 
 #include "context.cuh"
@@ -499,6 +501,13 @@ int32_t launch(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u3
     });
 }
 
+// bytes of the packed operands (the planes' workspace)
+size_t packed_bytes(u32 rows, u32 inner, u32 cols, u64 q) {
+    const int nb = (64 - __builtin_clzll(q - 1) + 7) / 8, ct = cols_per_tile(nb);
+    return (size_t)((inner + 31) / 32) * nb * 32 *
+           ((size_t)((rows + 127) / 128) * 128 + (size_t)((cols + ct - 1) / ct) * nb * ct);
+}
+
 // the tensor-core form covers every modulus; tile counts stay within int
 bool supported(u32 rows, u32 cols, u64 q) {
     const int nb = (64 - __builtin_clzll(q - 1) + 7) / 8;
@@ -561,12 +570,13 @@ __device__ __forceinline__ u32 residue(u32 lo, u32 hi, u32 r_lo, u32 r_hi, const
 
 // Both operands: per modulus 32-byte inner steps in the K-major core-matrix order.
 // A' [n][n_mt][n_kb][128 x 32]: one thread per (row, 16-deep run); B' [n][n_nt][n_kb][256 x 32]:
-// one thread per (column, 16-deep run). Threads [0, a_total) take A. Neighbouring threads take
-// neighbouring rows (columns), so a warp stores whole 128-byte core matrices.
+// one thread per (column, 16-deep run). Threads [0, a_total) take A; n_mt or n_nt = 0 leaves an
+// operand out. Rows of B lie ldb words apart. Neighbouring threads take neighbouring rows
+// (columns), so a warp stores whole 128-byte core matrices.
 __global__ void __launch_bounds__(256) k_rns_pack(const u64* __restrict__ A, const u64* __restrict__ B,
                                                   uint8_t* __restrict__ Ap, uint8_t* __restrict__ Bp, int rows,
-                                                  int inner, int cols, int n_mt, int n_nt, int n_kb, bool vec_a,
-                                                  const __grid_constant__ Params P) {
+                                                  int inner, int cols, size_t ldb, int n_mt, int n_nt, int n_kb,
+                                                  bool vec_a, const __grid_constant__ Params P) {
     const size_t runs = (size_t)2 * n_kb, a_total = (size_t)n_mt * 128 * runs, b_total = (size_t)n_nt * kN * runs;
     const size_t a_plane = (size_t)n_mt * n_kb * kATile, b_plane = (size_t)n_nt * n_kb * kBTile;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < a_total + b_total;
@@ -594,7 +604,7 @@ __global__ void __launch_bounds__(256) k_rns_pack(const u64* __restrict__ A, con
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
                 const int k = 16 * h + e;
-                v[e] = (c < cols && k < inner) ? B[(size_t)k * cols + c] : 0;
+                v[e] = (c < cols && k < inner) ? B[(size_t)k * ldb + c] : 0;
             }
             dst = Bp + ((size_t)(c / kN) * n_kb + (h >> 1)) * kBTile + ptc::core_off(c % kN, h & 1);
         }
@@ -768,10 +778,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == kMmaWarp) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
 }
 
-// C [rows][cols] from W: a thread combines four columns, stored through shared memory so
-// that a warp writes consecutive words.
+// C [rows][cols] (rows ldc words apart) from W: a thread combines four columns, stored through
+// shared memory so that a warp writes consecutive words.
 __global__ void __launch_bounds__(256) k_rns_combine(const uint8_t* __restrict__ W, u64* __restrict__ C, int rows,
-                                                     int cols, size_t plane, size_t pitch,
+                                                     int cols, size_t ldc, size_t plane, size_t pitch,
                                                      const __grid_constant__ Params P) {
     __shared__ __align__(16) u64 so[1024];
     const int c0 = blockIdx.x * 1024, c = c0 + 4 * threadIdx.x;
@@ -812,7 +822,7 @@ __global__ void __launch_bounds__(256) k_rns_combine(const uint8_t* __restrict__
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int o = threadIdx.x + 256 * e;
-            if (c0 + o < cols) C[(size_t)row * cols + c0 + o] = so[o];
+            if (c0 + o < cols) C[(size_t)row * ldc + c0 + o] = so[o];
         }
         __syncthreads();
     }
@@ -880,34 +890,67 @@ Params make_params(u32 inner, u64 q) {
     return P;
 }
 
+// Packed operands and W take P.n bytes an element of A, B and C, which for many outputs and a
+// short inner sum is far more than the planes' operands. The product is therefore made in slabs
+// of rt row tiles and ct column tiles whose workspace stays within what the planes would take,
+// or 2 GiB where that is less (a column slab's operand and its W for one row tile within half).
+struct Slabs {
+    int rt, ct;
+};
+Slabs slabs_for(u32 rows, u32 inner, u32 cols, u64 q, int n_mod) {
+    const int n_mt = (int)((rows + 127) / 128), n_nt = (int)((cols + kN - 1) / kN);
+    const size_t step = (size_t)n_mod * ((inner + 31) / 32) * 32;  // packed bytes of a row or column
+    const size_t budget = std::max((size_t)2 << 30, ptc::packed_bytes(rows, inner, cols, q));
+    auto even = [](int n, size_t most) {  // at most `most` (at least one) of n tiles, equal slabs
+        const int k = (int)std::min<size_t>((size_t)n, std::max<size_t>(1, most)), slabs = (n + k - 1) / k;
+        return (n + slabs - 1) / slabs;
+    };
+    Slabs s;
+    s.ct = even(n_nt, budget / 2 / (kN * (step + (size_t)128 * n_mod)));
+    const size_t b_bytes = (size_t)s.ct * kN * step;
+    s.rt = even(n_mt, (budget - b_bytes) / (128 * (step + (size_t)n_mod * s.ct * kN)));
+    return s;
+}
+
 int32_t run(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 cols, u64 q, cudaStream_t st) {
     const Params P = make_params(inner, q);
-    const int n_mt = (int)((rows + 127) / 128), n_nt = (int)((cols + kN - 1) / kN), n_kb = (int)((inner + 31) / 32);
+    const Slabs sl = slabs_for(rows, inner, cols, q, P.n);
+    const int n_kb = (int)((inner + 31) / 32);
+    const u32 slab_rows = (u32)sl.rt * 128, slab_cols = (u32)sl.ct * kN;
     int dev = 0, n_sm = 0;
     CKKS_CUDA_TRY(cudaGetDevice(&dev));
     CKKS_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    const size_t plane = (size_t)n_mt * 128 * n_nt * kN;
     return ptc::timed(dev, st, [&](int* err, auto packed) -> int32_t {
         Workspace<uint8_t> ap, bp, w;
         int32_t rc;
-        if ((rc = ap.alloc((size_t)P.n * n_mt * n_kb * kATile, st)) ||
-            (rc = bp.alloc((size_t)P.n * n_nt * n_kb * kBTile, st)) || (rc = w.alloc((size_t)P.n * plane, st)))
+        if ((rc = ap.alloc((size_t)P.n * sl.rt * n_kb * kATile, st)) ||
+            (rc = bp.alloc((size_t)P.n * sl.ct * n_kb * kBTile, st)) ||
+            (rc = w.alloc((size_t)P.n * slab_rows * slab_cols, st)))
             return rc;
-        const size_t threads = ((size_t)n_mt * 128 + (size_t)n_nt * kN) * 2 * n_kb, blocks = (threads + 255) / 256;
-        const size_t cap = (size_t)n_sm * 16;
-        k_rns_pack<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(lhs, rhs, ap.p, bp.p, (int)rows, (int)inner,
-                                                                            (int)cols, n_mt, n_nt, n_kb,
-                                                                            inner % 2 == 0 && ((uintptr_t)lhs & 15) == 0, P);
-        CKKS_CUDA_TRY(cudaGetLastError());
-        if ((rc = packed())) return rc;
         CKKS_CUDA_TRY(cudaFuncSetAttribute(k_rns_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-        const int n_tiles = n_mt * n_nt * P.n;
-        k_rns_gemm<<<n_tiles < n_sm ? n_tiles : n_sm, kThreads, kSmemBytes, st>>>(ap.p, bp.p, w.p, n_mt, n_nt, n_kb, P,
-                                                                                 err);
-        CKKS_CUDA_TRY(cudaGetLastError());
-        const dim3 g((cols + 1023) / 1024, rows < 65535 ? rows : 65535);
-        k_rns_combine<<<g, 256, 0, st>>>(w.p, out, (int)rows, (int)cols, plane, (size_t)n_nt * kN, P);
-        CKKS_CUDA_TRY(cudaGetLastError());
+        bool first = true;
+        for (u64 c0 = 0; c0 < cols; c0 += slab_cols)
+            for (u64 r0 = 0; r0 < rows; r0 += slab_rows) {
+                const u32 nr = (u32)std::min<u64>(slab_rows, rows - r0), nc = (u32)std::min<u64>(slab_cols, cols - c0);
+                const int n_mt = (int)((nr + 127) / 128), n_nt = (int)((nc + kN - 1) / kN), b_nt = r0 ? 0 : n_nt;
+                const u64* a = lhs + r0 * inner;
+                const size_t threads = ((size_t)n_mt * 128 + (size_t)b_nt * kN) * 2 * n_kb, blocks = (threads + 255) / 256;
+                const size_t cap = (size_t)n_sm * 16;
+                k_rns_pack<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(
+                    a, rhs + c0, ap.p, bp.p, (int)nr, (int)inner, (int)nc, cols, n_mt, b_nt, n_kb,
+                    inner % 2 == 0 && ((uintptr_t)a & 15) == 0, P);
+                CKKS_CUDA_TRY(cudaGetLastError());
+                if (first && (rc = packed())) return rc;
+                first = false;
+                const int n_tiles = n_mt * n_nt * P.n;
+                k_rns_gemm<<<n_tiles < n_sm ? n_tiles : n_sm, kThreads, kSmemBytes, st>>>(ap.p, bp.p, w.p, n_mt, n_nt,
+                                                                                         n_kb, P, err);
+                CKKS_CUDA_TRY(cudaGetLastError());
+                const dim3 g((nc + 1023) / 1024, nr < 65535 ? nr : 65535);
+                k_rns_combine<<<g, 256, 0, st>>>(w.p, out + r0 * cols + c0, (int)nr, (int)nc, cols,
+                                                 (size_t)n_mt * 128 * n_nt * kN, (size_t)n_nt * kN, P);
+                CKKS_CUDA_TRY(cudaGetLastError());
+            }
         return CKKS_OK;
     });
 }
@@ -939,7 +982,11 @@ int32_t ckks_park_mod_pp_mm_with_backend(const uint64_t* lhs, const uint64_t* rh
     if (backend == CKKS_PARK_TENSOR_CORES) {
         CKKS_CHECK_ARG(tc_ok, "ckks_park_mod_pp_mm: the tensor-core backend needs a compute capability 10.0 device "
                               "and fewer than 2^31 output tiles");
-        if (rns::worthwhile(rows, inner, cols, modulus)) return rns::run(lhs, rhs, out, rows, inner, cols, modulus, st);
+        if (rns::worthwhile(rows, inner, cols, modulus)) {
+            // out of memory before any output is written: the planes may still fit
+            const int32_t rc = rns::run(lhs, rhs, out, rows, inner, cols, modulus, st);
+            if (rc != CKKS_ERR_OOM) return rc;
+        }
         return ptc::run(lhs, rhs, out, rows, inner, cols, modulus, st);
     }
     CKKS_CHECK_ARG(backend == CKKS_PARK_CUDA_CORES, "ckks_park_mod_pp_mm: unknown backend");

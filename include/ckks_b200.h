@@ -276,22 +276,24 @@ int32_t ckks_ksk_destroy(ckks_ksk* key);
 int32_t ckks_park_mod_pp_mm(const uint64_t* lhs, const uint64_t* rhs, uint64_t* out, uint32_t rows, uint32_t inner,
                             uint32_t cols, uint64_t modulus, void* stream);
 /* park_matrix_mul_with_backend (ccmm/park.rs:1643-1655) for the device
- * backends: AUTO takes the tensor cores (unsigned 8-bit products of the
- * residues' bytes against byte-split weights 2^(8i) rhs mod q, summed exactly
- * in 32 bits; the call waits for its status word, so it returns with the
- * stream drained) and otherwise the CUDA cores (exact 192-bit sums, stream-
- * ordered). Both return the same words. A backend that cannot run returns
- * CKKS_ERR_BAD_ARG; a tensor-core pipeline wait that timed out returns
- * CKKS_ERR_TIMEOUT. The tensor cores take stream-ordered workspace for the
- * packed operands, about nb * rows * inner + nb^2 * inner * cols bytes (nb =
- * bytes of modulus - 1, rows, inner and cols rounded up to their tiles); when
- * it does not fit the call returns CKKS_ERR_OOM and leaves the choice of the
- * CUDA-core backend to the caller. */
+ * backends: AUTO takes the tensor cores (unsigned 8-bit products summed exactly
+ * in 32 bits, of the residues' bytes against byte-split weights 2^(8i) rhs mod
+ * q, or, for wider moduli below 2^62, of both operands modulo up to 20 coprime
+ * moduli of at most 256; the call waits for its status word, so it returns with
+ * the stream drained) and otherwise the CUDA cores (exact 192-bit sums, stream-
+ * ordered). All return the same words. A backend that cannot run returns CKKS_ERR_BAD_ARG; a tensor-core pipeline
+ * wait that timed out returns CKKS_ERR_TIMEOUT. The tensor cores take stream-
+ * ordered workspace: the packed operands of the byte form, about nb * rows *
+ * inner + nb^2 * inner * cols bytes (nb = bytes of modulus - 1, rows, inner and
+ * cols rounded up to their tiles), or at most the larger of that and 2 GiB for
+ * the residue form, which works in slabs. When the byte form's does not fit
+ * either the call returns CKKS_ERR_OOM and leaves the choice of the CUDA-core
+ * backend to the caller. */
 enum { CKKS_PARK_AUTO = 0, CKKS_PARK_TENSOR_CORES = 1, CKKS_PARK_CUDA_CORES = 2 };
 int32_t ckks_park_mod_pp_mm_with_backend(const uint64_t* lhs, const uint64_t* rhs, uint64_t* out, uint32_t rows,
                                          uint32_t inner, uint32_t cols, uint64_t modulus, int32_t backend,
                                          void* stream);
-/* CUDA-event times (ms) of the byte packing and of the GEMM launches of this
+/* CUDA-event times (ms) of the (first slab's) packing and of the rest of this
  * thread's last tensor-core Park call; CKKS_ERR_BAD_ARG before the first. */
 int32_t ckks_park_last_timing(float* pack_ms, float* gemm_ms);
 int32_t ckks_park_mod_pp_mm_host(const uint64_t* lhs, const uint64_t* rhs, uint64_t* out, uint32_t rows,

@@ -40,3 +40,37 @@ def test_four_byte_modulus_above_the_size_line(cuda):
     import torch
     assert torch.equal(cb.park_mod_pp_mm(a, b, q, backend="tensor_cores"),
                        cb.park_mod_pp_mm(a, b, q, backend="cuda_cores"))
+
+
+def random(rows, cols, q, seed):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.empty((rows, cols), dtype=torch.int64, device="cuda").random_(0, q, generator=gen)
+
+
+def peak_workspace(call):
+    """Device bytes that a call takes from the stream-ordered pool at its peak."""
+    import torch
+    from cuda.bindings import driver, runtime as rt
+    torch.cuda.synchronize()
+    err, pool = rt.cudaDeviceGetDefaultMemPool(torch.cuda.current_device())
+    assert int(err) == 0
+    attr = rt.cudaMemPoolAttr
+    before = int(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemCurrent)[1])
+    assert int(rt.cudaMemPoolSetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh, driver.cuuint64_t(0))[0]) == 0
+    out = call()
+    torch.cuda.synchronize()
+    return out, int(rt.cudaMemPoolGetAttribute(pool, attr.cudaMemPoolAttrUsedMemHigh)[1]) - before
+
+
+# row slabs, column slabs and both: residues of the whole product beyond 2 GiB
+@pytest.mark.parametrize("shape", [(12000, 1030, 11000), (200, 1, 500000), (600, 1, 500000)])
+def test_products_beyond_the_workspace_limit_in_slabs(cuda, shape):
+    import torch
+    q = (1 << 60) - 93
+    (r, k, c), limit = shape, 2 << 30
+    a, b = random(r, k, q, 1), random(k, c, q, 2)
+    got, peak = peak_workspace(lambda: cb.park_mod_pp_mm(a, b, q, backend="tensor_cores"))
+    packed = 8 * k * (r + 8 * c)  # of the byte planes, which may be the larger limit
+    assert peak < max(limit, 1.2 * packed) + (64 << 20), peak
+    assert torch.equal(got, cb.park_mod_pp_mm(a, b, q, backend="cuda_cores"))

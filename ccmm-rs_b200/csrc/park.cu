@@ -33,8 +33,8 @@
 // reciprocals (each below the true one by under 2^-27: the sum is off by under 2^-14).
 // Packing takes two byte dot products an element and modulus; the GEMM is the persistent
 // kernel below with N = 256 and one accumulator, storing w_i as bytes; one kernel combines
-// the n_mod bytes of an output, in slabs of the product whose workspace is bounded. n = 4096,
-// 35-bit q: packing 0.17 ms, GEMM 0.54 ms (2.80 POP/s,
+// the n_mod bytes of an output, in slabs of the product whose workspace is bounded. Chosen by
+// estimated times (worthwhile). n = 4096, 35-bit q: packing 0.17 ms, GEMM 0.54 ms (2.80 POP/s,
 // 88 % of twice the bf16 rate: the tensor pipe bounds it), combining 0.12 ms; the byte planes
 // took 0.26 and 1.24 ms.
 //
@@ -779,14 +779,20 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // C [rows][cols] (rows ldc words apart) from W: a thread combines four columns, stored through
-// shared memory so that a warp writes consecutive words.
+// shared memory so that a warp writes consecutive words. A block of 256 threads takes 4 X columns
+// of 256 / X rows (narrow outputs several rows: 65536 x 32 x 256, 60 bits, 0.63 -> 0.44 ms).
+template <int X>
 __global__ void __launch_bounds__(256) k_rns_combine(const uint8_t* __restrict__ W, u64* __restrict__ C, int rows,
                                                      int cols, size_t ldc, size_t plane, size_t pitch,
                                                      const __grid_constant__ Params P) {
-    __shared__ __align__(16) u64 so[1024];
-    const int c0 = blockIdx.x * 1024, c = c0 + 4 * threadIdx.x;
-    for (int row = blockIdx.y; row < rows; row += gridDim.y) {
-        if (c < cols) {  // pitch is a multiple of 256: the four bytes are inside the row
+    __shared__ __align__(16) u64 so_[1024];
+    constexpr int kRows = 256 / X;
+    const int tx = threadIdx.x % X, ty = threadIdx.x / X, c0 = blockIdx.x * 4 * X, c = c0 + 4 * tx;
+    u64* so = so_ + ty * 4 * X;
+    for (int r0 = blockIdx.y * kRows; r0 < rows; r0 += gridDim.y * kRows) {
+        const int row = r0 + ty;
+        const bool on = kRows == 1 || row < rows;
+        if (on && c < cols) {  // pitch is a multiple of 256: the four bytes are inside the row
             const uint8_t* src = W + (size_t)row * pitch + c;
             u32 k[4] = {0, 0, 0, 0};
             u64 lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
@@ -815,14 +821,14 @@ __global__ void __launch_bounds__(256) k_rns_combine(const uint8_t* __restrict__
                 u64 x = mul_shoup_lazy(hi[e], P.r32, P.r32q, P.q) + lo[e];  // below 2 q + 2^45
                 x -= __umul64hi(x, P.mu) * P.q;
                 x = x >= P.q ? x - P.q : x;
-                so[4 * threadIdx.x + e] = x >= P.q ? x - P.q : x;
+                so[4 * tx + e] = x >= P.q ? x - P.q : x;
             }
         }
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int o = threadIdx.x + 256 * e;
-            if (c0 + o < cols) C[(size_t)row * ldc + c0 + o] = so[o];
+            const int o = tx + X * e;
+            if (on && c0 + o < cols) C[(size_t)row * ldc + c0 + o] = so[o];
         }
         __syncthreads();
     }
@@ -839,15 +845,27 @@ int moduli_for(u32 inner, u64 q) {
     return 0;
 }
 
-// Where the residue system is faster than the byte planes, by moduli of nb bytes (ms, planes
-// against residues, n x n x n): nb <= 3 has at most 9 products against 6 to 9 and an extra
-// combining pass; nb = 4 (32 bits) n = 1024 0.096 / 0.102, n = 2048 0.239 / 0.205, n = 4096
-// 1.052 / 0.834; nb = 5 (35 bits) n = 256 0.084 / 0.078, n = 4096 1.542 / 0.894; nb = 8
-// (60 bits) n = 64 0.096 / 0.082, n = 4096 3.653 / 1.399.
+// Whether the residue system takes less time than the byte planes (moduli of at least 4 bytes;
+// narrower ones have at most 9 products against 6 to 9 and an extra combining pass), by estimates
+// (ps) fitted to both on a B200 (seven moduli of 30 to 60 bits, 46 shapes, within about 10 %).
+// An output of the planes costs the epilogue of its nb accumulators or its nb^2 products,
+// whichever is longer; one of the residues costs n bytes written and read back and n products,
+// with columns padded to 256. Packing an element of lhs or rhs costs the planes 4 or 8 ps more,
+// a call 6 us (two packing launches). ms, planes / residues: 35 bits, 4096 x inner x 4096: inner = 64
+// 0.182 / 0.304, 512 0.305 / 0.345, 1024 0.470 / 0.418, 4096 1.59 / 0.92; 16384 x 64 x 16384 1.80 / 3.95;
+// 60 bits, 4096 x 64 x 4096 0.40 / 0.43, 4096^3 3.68 / 1.41, 65536 x 32 x 16 0.120 / 0.335. Moduli of
+// 4 bytes below 2^31 products differ by a few us either way and keep the planes.
 bool worthwhile(u32 rows, u32 inner, u32 cols, u64 q) {
-    if (q <= (1ull << 24) || q >= (1ull << 62) || inner > (u32)kMaxInner || !moduli_for(inner, q)) return false;
-    if (q <= (1ull << 32) && (double)rows * inner * cols < 2147483648.0) return false;
-    return (u64)((rows + 127) / 128) * ((cols + kN - 1) / kN) < (1ull << 26);
+    if (q <= (1ull << 24) || q >= (1ull << 62) || inner > (u32)kMaxInner) return false;
+    const double r = rows, k = inner, c = cols;
+    if (q <= (1ull << 32) && r * k * c < 2147483648.0) return false;
+    const int n = moduli_for(inner, q), nb = (64 - __builtin_clzll(q - 1) + 7) / 8, ct = ptc::cols_per_tile(nb);
+    if (!n) return false;
+    const u64 n_mt = (rows + 127) / 128, n_nt = (cols + kN - 1) / kN;
+    if (n_mt * n_nt >= (1ull << 26)) return false;
+    const double out = 128.0 * n_mt, planes_out = std::max(nb <= 5 ? 6.5 : 18.0, 0.87e-3 * nb * nb * k);
+    const double planes = out * ((cols + ct - 1) / ct * ct) * planes_out + 4 * r * k + 8 * k * c + 6e6;
+    return out * n_nt * kN * (2.5 + n * (0.95 + 0.55e-3 * k)) < planes;
 }
 
 Params make_params(u32 inner, u64 q) {
@@ -946,9 +964,15 @@ int32_t run(const u64* lhs, const u64* rhs, u64* out, u32 rows, u32 inner, u32 c
                 k_rns_gemm<<<n_tiles < n_sm ? n_tiles : n_sm, kThreads, kSmemBytes, st>>>(ap.p, bp.p, w.p, n_mt, n_nt,
                                                                                          n_kb, P, err);
                 CKKS_CUDA_TRY(cudaGetLastError());
-                const dim3 g((nc + 1023) / 1024, nr < 65535 ? nr : 65535);
-                k_rns_combine<<<g, 256, 0, st>>>(w.p, out + r0 * cols + c0, (int)nr, (int)nc, cols,
-                                                 (size_t)n_mt * 128 * n_nt * kN, (size_t)n_nt * kN, P);
+                u32 x = 32;  // threads a row
+                while (x < 256 && 4 * x < nc) x *= 2;
+                const dim3 g((nc + 4 * x - 1) / (4 * x), std::min<u32>((nr * x + 255) / 256, 65535));
+                auto* combine = x == 32    ? k_rns_combine<32>
+                                : x == 64  ? k_rns_combine<64>
+                                : x == 128 ? k_rns_combine<128>
+                                           : k_rns_combine<256>;
+                combine<<<g, 256, 0, st>>>(w.p, out + r0 * cols + c0, (int)nr, (int)nc, cols,
+                                           (size_t)n_mt * 128 * n_nt * kN, (size_t)n_nt * kN, P);
                 CKKS_CUDA_TRY(cudaGetLastError());
             }
         return CKKS_OK;

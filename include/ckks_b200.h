@@ -278,10 +278,11 @@ int32_t ckks_park_mod_pp_mm(const uint64_t* lhs, const uint64_t* rhs, uint64_t* 
 /* park_matrix_mul_with_backend (ccmm/park.rs:1643-1655) for the device
  * backends: AUTO takes the tensor cores (unsigned 8-bit products summed exactly
  * in 32 bits, of the residues' bytes against byte-split weights 2^(8i) rhs mod
- * q, or, for wider moduli below 2^62, of both operands modulo up to 20 coprime
- * moduli of at most 256; the call waits for its status word, so it returns with
- * the stream drained) and otherwise the CUDA cores (exact 192-bit sums, stream-
- * ordered). All return the same words. A backend that cannot run returns CKKS_ERR_BAD_ARG; a tensor-core pipeline
+ * q, or, for moduli above 2^24 and below 2^62 where that is faster, of both
+ * operands modulo up to 20 coprime moduli of at most 256; the call waits for
+ * its status word, so it returns with the stream drained) and otherwise the
+ * CUDA cores (exact 192-bit sums, stream-ordered). All return the same words.
+ * A backend that cannot run returns CKKS_ERR_BAD_ARG; a tensor-core pipeline
  * wait that timed out returns CKKS_ERR_TIMEOUT. The tensor cores take stream-
  * ordered workspace: the packed operands of the byte form, about nb * rows *
  * inner + nb^2 * inner * cols bytes (nb = bytes of modulus - 1, rows, inner and

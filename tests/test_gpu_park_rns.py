@@ -74,3 +74,23 @@ def test_products_beyond_the_workspace_limit_in_slabs(cuda, shape):
     packed = 8 * k * (r + 8 * c)  # of the byte planes, which may be the larger limit
     assert peak < max(limit, 1.2 * packed) + (64 << 20), peak
     assert torch.equal(got, cb.park_mod_pp_mm(a, b, q, backend="cuda_cores"))
+
+
+# where writing and reading a residue per modulus and output outweighs the products saved
+@pytest.mark.parametrize("bits,shape", [(35, (4096, 64, 4096)), (35, (65536, 32, 16)), (47, (20000, 32, 16)),
+                                        (56, (20000, 33, 9)), (60, (20000, 32, 16))])
+def test_short_inner_sums_take_the_byte_planes(cuda, bits, shape):
+    import torch
+    q = (1 << bits) - 115
+    a, b = random(*shape[:2], q, 3), random(*shape[1:], q, 4)
+    got, peak = peak_workspace(lambda: cb.park_mod_pp_mm(a, b, q, backend="tensor_cores"))
+    assert peak < 8 * shape[0] * max(shape[2], 256)  # the residue form takes at least 11 bytes an output
+    assert torch.equal(got, cb.park_mod_pp_mm(a, b, q, backend="cuda_cores"))
+
+
+@pytest.mark.parametrize("bits", [40, 47, 56, 61])  # five to eight bytes
+def test_chunked_byte_planes_of_wide_moduli(oracle, cuda, bits):
+    """Inner sums beyond the residue system's: several plane launches that add their residues."""
+    rng = np.random.default_rng(bits)
+    check(oracle, rng.integers(0, 2**64, (3, 33100), dtype=np.uint64), rng.integers(0, 2**64, (33100, 5), dtype=np.uint64),
+          (1 << bits) - 115)

@@ -162,15 +162,16 @@ _raw_stream = None
 
 def _stream(stream):
     """The caller's stream, or torch's current one of the current device: asked by its raw
-    handle, since building a Stream object on every call costs more than a launch."""
+    handle where torch has that call (not public), since building a Stream object on every
+    call costs more than a launch."""
     global _raw_stream
     if stream is not None:
         return stream
     if _raw_stream is None:
         import torch
         torch.cuda.current_stream()  # initialises CUDA
-        get, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
-        _raw_stream = lambda: get(device())  # noqa: E731
+        get, device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+        _raw_stream = (lambda: get(device())) if get and device else lambda: torch.cuda.current_stream().cuda_stream
     return _raw_stream()
 
 

@@ -10,13 +10,8 @@ from ckks_b200.params import chain
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("q_bits", [(50, 50), (55, 40), (30, 49)])
-@pytest.mark.parametrize("m,k,n", [(7, 1, 2), (8, 3, 17), (9, 9, 1), (31, 2, 3), (32, 5, 33), (33, 64, 2)])
-def test_tensor_cores_equal_cuda_cores(cuda, q_bits, m, k, n):
+def compare(ctx, key, q, m, k, n):
     import torch
-    q, _ = chain(1 << 8, q_bits)
-    ctx = cb.Context(8, q)
-    key = cb.KeySwitchKey.relin_generate(ctx, len(q), 20, np.random.default_rng(2).integers(-1, 2, ctx.n), seed=5)
     gen = torch.Generator(device="cuda").manual_seed(m + k + n)
 
     def matrix(*lead):
@@ -32,3 +27,22 @@ def test_tensor_cores_equal_cuda_cores(cuda, q_bits, m, k, n):
     assert ctx.last_mac_path == "tensor_cores"
     ctx.tensor_cores = False
     assert torch.equal(got, cb.matmul_structured(ctx, key, a, b, m, k, n))
+
+
+@pytest.mark.parametrize("q_bits", [(50, 50), (55, 40), (30, 49)])
+@pytest.mark.parametrize("m,k,n", [(7, 1, 2), (8, 3, 17), (9, 9, 1), (31, 2, 3), (32, 5, 33), (33, 64, 2)])
+def test_tensor_cores_equal_cuda_cores(cuda, q_bits, m, k, n):
+    q, _ = chain(1 << 8, q_bits)
+    ctx = cb.Context(8, q)
+    key = cb.KeySwitchKey.relin_generate(ctx, len(q), 20, np.random.default_rng(2).integers(-1, 2, ctx.n), seed=5)
+    compare(ctx, key, q, m, k, n)
+
+
+# an A of more than 2^28 words is transformed and written in several calls (60 entries each here):
+# whole pairs of inner indices a call, odd inner sizes, rows below 8, fewer entries than a pair
+@pytest.mark.parametrize("m,k,n", [(20, 5, 1), (7, 19, 2), (64, 3, 1), (29, 4, 1), (1, 64, 1)])
+def test_images_written_in_several_calls(cuda, m, k, n):
+    q, _ = chain(1 << 17, (50,) * 17)
+    ctx = cb.Context(17, q)
+    key = cb.KeySwitchKey.relin_generate(ctx, len(q), 45, np.random.default_rng(2).integers(-1, 2, ctx.n), seed=5)
+    compare(ctx, key, q, m, k, n)

@@ -205,11 +205,17 @@ k_fwd1(const void* __restrict__ in_, u64* __restrict__ out,
         const int c = tid & (C - 1), i0 = tid >> log_c;
         u64 x[S::R1];
         if (kDigits) {
-            const i64* in = (const i64*)in_ + ((size_t)blockIdx.z << (LOG_M + log_b));
+            // one branch outside the loops: with a choice in every step each load waited for the
+            // digit before it (four 60-bit limbs of N = 2^13, 840 digits: 311 -> 201 us)
+            const i64* in = (const i64*)in_ + ((size_t)blockIdx.z << (LOG_M + log_b)) + c0 + c + ((size_t)i0 << log_b);
 #pragma unroll
-            for (int e = 0; e < S::R1; ++e) {
-                const i64 d = in[c0 + c + ((size_t)(i0 + S::R2 * e) << log_b)];
-                x[e] = small ? lift_small(d, q) : lift_digit(d, q, T.mu_hi);
+            for (int e = 0; e < S::R1; ++e) x[e] = (u64)in[(size_t)(S::R2 * e) << log_b];
+            if (small) {
+#pragma unroll
+                for (int e = 0; e < S::R1; ++e) x[e] = lift_small((i64)x[e], q);
+            } else {
+#pragma unroll
+                for (int e = 0; e < S::R1; ++e) x[e] = lift_digit((i64)x[e], q, T.mu_hi);
             }
         } else {
             const u64* in = (const u64*)in_ + base;

@@ -1357,9 +1357,10 @@ def bench_park_gpu(args, world, rank, local):
             "config": park_config(n),
             "roofline": {"bound": "tensor", "achieved": achieved, "unit": "TOP/s (INT8)", "peak": i8_peak,
                          "frac": achieved / i8_peak if i8_peak else None,
-                         # packed operands and residues of the product once each, and the product
-                         "traffic": (4.0 * n_mod + 8.0) * n * n,
-                         "traffic_source": "algorithmic bytes of the product and combining passes",
+                         # DRAM bytes of the two kernels at n = 4096 (read 369.2 + 184.6 MB, written
+                         # 160.8 + 71.8 MB), scaled by n^2 like the arrays they move
+                         "traffic": 786.4e6 * (n / 4096.0) ** 2,
+                         "traffic_source": "ncu DRAM counters of the n=4096 launches, scaled by (n/4096)^2",
                          "kernel": "k_rns_gemm + k_rns_combine (INT8 tcgen05 products of %d residues)" % n_mod,
                          "kernel_ms": gemm, "rest_of_step_ms": (ms_max / args.steps) - gemm,
                          "peak_source": "2 x bf16 dense (%s %s)" % (bf16_kind, bf16),
@@ -1374,10 +1375,14 @@ def bench_park_gpu(args, world, rank, local):
             "gpu_launches": 3 * args.steps, "clocks": clk}
 
 
+# csrc/park.cu, rns::kModuli
+PARK_MODULI = (256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193, 191, 181, 179, 173)
+
+
 def park_moduli(n, q):
     """Moduli of the residue-system product (csrc/park.cu, rns::moduli_for)."""
     need, have = 1.05 + np.log2(n) + 2.0 * np.log2(q - 1), 0.0
-    for i, m in enumerate((256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193)):
+    for i, m in enumerate(PARK_MODULI):
         have += np.log2(m)
         if have > need:
             return i + 1

@@ -1189,9 +1189,9 @@ constexpr bool kFuseModDown = CKKS_FUSE_MODDOWN != 0;
 
 // (ciphertext, key) pairs of a group up to which the MAC may run on the FP64 pipe
 // (mac_f64.cuh): where it is the faster one, macf::cheaper_than_tc, and where the keys' packed
-// set does not fit and more than 4 ciphertexts share a key slice (16 x 11 pairs at N = 2^16,
-// 24 + 3 limbs: 28.8 ms against 36.7 with 16 x 12 on the CUDA cores; 4 x 24: 20.4 against 16.8).
-// The measurements of both end at 160 pairs.
+// set does not fit and more than 4 ciphertexts share a key slice (FP64 against CUDA cores at
+// N = 2^16, 24 + 3 limbs: 16 x 12 pairs 28.8 / 36.7 ms, 4 x 24 20.4 / 16.8).
+// The rule's measurements end at 160 pairs.
 constexpr size_t kF64MacPairs = 160;
 
 // Hoisted hybrid rotations of n_ct ciphertexts by n_keys Galois keys (bounded

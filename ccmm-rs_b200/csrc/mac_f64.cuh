@@ -22,8 +22,8 @@
 // for 32 keys and for 1 as for 16 ciphertexts (its cost is per item of 4 slots x
 // 4 digits, about 1,380 cycles); here the FMAs follow the pairs: 4 per product at
 // 64 a clock and SM. The sums take 96 registers a thread, so four warps a scheduler
-// cover the FMA and shared-memory latencies: the FP64 pipe is 33 % active, with no
-// single stall above a quarter of the cycles. Leaving out the splitting (13 % of the
+// cover the FMA and shared-memory latencies: the FP64 pipe is 29 % active (34 % in the
+// three-piece form), with no single stall above a third of the issue slots' wait. Leaving out the splitting (13 % of the
 // time), the fetches (5 %) or the final reductions (5 %) in timing-only copies shows
 // the FMA loop itself holds the rest. Two-digit unrolling (+4 %), 255 registers at
 // half the warps (+35 %) and row-wise bulk copies (85 cycles a copy: 2.4x the time)

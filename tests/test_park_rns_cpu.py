@@ -2,7 +2,9 @@
 restated on the CPU: the number of moduli, the quotient k from 2^27-scaled reciprocals and
 the final combination give the exact product modulo q, at the extremes of the sums too."""
 import math
+import os
 import random
+import re
 
 import pytest
 
@@ -30,6 +32,14 @@ def combine(w, mods, q):
     hi = sum(wi * ((M // m % q) >> 32) for wi, m in zip(w, mods)) + k * (nm >> 32)
     assert lo < 1 << 45 and hi < 1 << 45 and 2 * q + lo < 1 << 64
     return k, (lo + (hi << 32)) % q
+
+
+def test_one_list_of_moduli():
+    """The kernels', the bench's and this file's."""
+    root = os.path.join(os.path.dirname(__file__), "..")
+    for path, name in (("ccmm-rs_b200/csrc/park.cu", r"kModuli\[kMaxMod\] = \{"), ("bench.py", r"PARK_MODULI = \(")):
+        text = open(os.path.join(root, path)).read()
+        assert [int(x) for x in re.search(name + r"([\d,\s]+)[})]", text).group(1).split(",")] == MODULI, path
 
 
 def test_moduli_are_coprime_bytes():
